@@ -33,18 +33,19 @@ template <class R> GMT_HD void fast_speed_adj(const Q9<R>& q, R gamma, R bn, R c
     const R dm_b = sd > R(0) ? t_b * (R(0.5) / sd) : R(0);
     const R disc_b = dm_b * sel_ge(disc, R(0));
     d2_b += disc_b * R(2) * d2;
-    R c2_b = -disc_b * (bn * bn / rho);
-    bnb += -disc_b * c2 * R(2) * bn / rho;
-    R rho_b = disc_b * (c2 * bn * bn / (rho * rho));
+    const R ir = R(1) / rho, w = bn * bn * ir;
+    R c2_b = -disc_b * w;
+    bnb += -disc_b * c2 * R(2) * bn * ir;
+    R rho_b = disc_b * c2 * w * ir;
     const R b2_b = R(0.5) * d2_b;
     c2_b += R(0.5) * d2_b;
-    const R bsq_b = b2_b / rho;
-    rho_b += -b2_b * b2 / rho;
+    const R bsq_b = b2_b * ir;
+    rho_b += -b2_b * b2 * ir;
     qb.v[5] += bsq_b * R(2) * q.v[5];
     qb.v[6] += bsq_b * R(2) * q.v[6];
     qb.v[7] += bsq_b * R(2) * q.v[7];
-    qb.v[4] += c2_b * gamma / rho;
-    rho_b += -c2_b * c2 / rho;
+    qb.v[4] += c2_b * gamma * ir;
+    rho_b += -c2_b * c2 * ir;
     qb.v[0] += rho_b;
 }
 
@@ -55,7 +56,8 @@ template <class R> GMT_HD void phys_flux_x_adj(const Q9<R>& q, R gamma, const Q9
     const R b2 = bx * bx + by * by + bz * bz;
     const R ptot = p + R(0.5) * b2;
     const R vsq = vx * vx + vy * vy + vz * vz;
-    const R E = p / (gamma - R(1)) + R(0.5) * rho * vsq + R(0.5) * b2;
+    const R igm1 = R(1) / (gamma - R(1));
+    const R E = p * igm1 + R(0.5) * rho * vsq + R(0.5) * b2;
     const R vdotb = vx * bx + vy * by + vz * bz;
     const R f0 = fb.v[0], f1 = fb.v[1], f2 = fb.v[2], f3 = fb.v[3], f4 = fb.v[4], f6 = fb.v[6], f7 = fb.v[7];
     R rho_b = f0 * vx + f1 * vx * vx + f2 * vx * vy + f3 * vx * vz;
@@ -70,7 +72,7 @@ template <class R> GMT_HD void phys_flux_x_adj(const Q9<R>& q, R gamma, const Q9
     R bz_b = -f3 * bx + f7 * vx;
     vx_b += vdotb_b * bx; vy_b += vdotb_b * by; vz_b += vdotb_b * bz;
     bx_b += vdotb_b * vx; by_b += vdotb_b * vy; bz_b += vdotb_b * vz;
-    R p_b = E_b / (gamma - R(1)) + ptot_b;
+    R p_b = E_b * igm1 + ptot_b;
     rho_b += E_b * R(0.5) * vsq;
     vx_b += E_b * rho * vx; vy_b += E_b * rho * vy; vz_b += E_b * rho * vz;
     const R b2_b = R(0.5) * E_b + R(0.5) * ptot_b;
@@ -168,341 +170,272 @@ GMT_HD void hll_x_adj(const Q9<R>& L, const Q9<R>& Rr, R gamma, R bn, const Q9<R
     fast_speed_adj(Rr, gamma, bn, -aR_b + bR_b, Rb, bnb);
 }
 
-// HLLD star state (hlld_star) and its reverse
-template <class R>
-GMT_HD void hlld_star_adj(R d, R u, R v, R w, R by, R bz, R S, R SM, R bn, R vy_b, R vz_b, R byS_b, R bzS_b, R& d_b,
-                          R& u_b, R& v_b, R& w_b, R& by_b, R& bz_b, R& S_b, R& SM_b, R& bn_b) {
-    const R a = S - u, b = S - SM;
-    const R denK = d * a * b - bn * bn;
-    if (rabs(denK) < R(1e-12)) {
-        v_b += vy_b; w_b += vz_b; by_b += byS_b; bz_b += bzS_b;
-        return;
+// HLLD star state of one side (hlld_star) and its reverse; `ik` is 1 / denK, `degen` the branch taken
+template <class R> struct HStar {
+    R vy, vz, by, bz, ik;
+    bool degen;
+};
+template <class R> GMT_HD HStar<R> hstar(R d, R u, R v, R w, R by, R bz, R S, R SM, R bn) {
+    HStar<R> s;
+    const R denK = d * (S - u) * (S - SM) - bn * bn;
+    s.degen = rabs(denK) < R(1e-12);
+    s.vy = v; s.vz = w; s.by = by; s.bz = bz; s.ik = R(0);
+    if (!s.degen) {
+        s.ik = R(1) / denK;
+        const R fac = bn * (SM - u) * s.ik, t = (d * (S - u) * (S - u) - bn * bn) * s.ik;
+        s.vy = v - by * fac;
+        s.vz = w - bz * fac;
+        s.by = by * t;
+        s.bz = bz * t;
     }
-    const R fac = bn * (SM - u) / denK;
-    const R num = d * a * a - bn * bn;
-    const R byS = by * num / denK, bzS = bz * num / denK;
+    return s;
+}
+template <class R>
+GMT_HD void hstar_adj(R d, R u, R by, R bz, R S, R SM, R bn, const HStar<R>& s, R vy_b, R vz_b, R byS_b, R bzS_b,
+                      R& d_b, R& u_b, R& v_b, R& w_b, R& by_b, R& bz_b, R& S_b, R& SM_b, R& bn_b) {
     v_b += vy_b;
     w_b += vz_b;
-    by_b += -vy_b * fac + byS_b * num / denK;
-    bz_b += -vz_b * fac + bzS_b * num / denK;
-    const R fac_b = -vy_b * by - vz_b * bz;
-    const R num_b = (byS_b * by + bzS_b * bz) / denK;
-    R denK_b = -(byS_b * byS + bzS_b * bzS) / denK - fac_b * fac / denK;
-    bn_b += fac_b * (SM - u) / denK;
-    SM_b += fac_b * bn / denK;
-    u_b += -fac_b * bn / denK;
-    d_b += num_b * a * a + denK_b * a * b;
+    if (s.degen) {
+        by_b += byS_b; bz_b += bzS_b;
+        return;
+    }
+    const R a = S - u, b = S - SM, ik = s.ik;
+    const R fac = bn * (SM - u) * ik, t = (d * a * a - bn * bn) * ik;
+    by_b += -vy_b * fac + byS_b * t;
+    bz_b += -vz_b * fac + bzS_b * t;
+    const R fac_b = -(vy_b * by + vz_b * bz) * ik;        // of the numerators
+    const R num_b = (byS_b * by + bzS_b * bz) * ik;
+    const R denK_b = -(num_b * t + fac_b * fac);
+    bn_b += fac_b * (SM - u) - R(2) * bn * (num_b + denK_b);
+    d_b += (num_b * a + denK_b * b) * a;
     const R a_b = num_b * R(2) * d * a + denK_b * d * b;
     const R b_b = denK_b * d * a;
-    bn_b += -num_b * R(2) * bn - denK_b * R(2) * bn;
+    SM_b += fac_b * bn - b_b;
+    u_b += -fac_b * bn - a_b;
     S_b += a_b + b_b;
-    u_b += -a_b;
-    SM_b += -b_b;
 }
 
-// one side of the HLLD fan: the side's primitive state and its star quantities
-template <class R> struct HSide {
-    R d, u, v, w, p, by, bz, E, pt, S;
-    R vys, vzs, bys, bzs, vdotb, vdotbs, Es;
-};
-template <class R> struct HSideB {
-    R d, u, v, w, p, by, bz, E, pt, S, vys, vzs, bys, bzs, vdotbs, Es;
-};
-
-template <class R> GMT_HD void hside_zero(HSideB<R>& b) {
-    b.d = b.u = b.v = b.w = b.p = b.by = b.bz = b.E = b.pt = b.S = R(0);
-    b.vys = b.vzs = b.bys = b.bzs = b.vdotbs = b.Es = R(0);
-}
-
-template <class R> GMT_HD void hside_star(HSide<R>& s, R SM, R pts, R bn) {
-    hlld_star(s.d, s.u, s.v, s.w, s.by, s.bz, s.S, SM, bn, s.vys, s.vzs, s.bys, s.bzs);
-    s.vdotb = s.u * bn + s.v * s.by + s.w * s.bz;
-    s.vdotbs = SM * bn + s.vys * s.bys + s.vzs * s.bzs;
-    s.Es = ((s.S - s.u) * s.E - s.pt * s.u + pts * SM + bn * (s.vdotb - s.vdotbs)) / (s.S - SM);
-}
-
-// reverse of hside_star: from b.vys..b.bzs, b.vdotbs, b.Es to the side inputs, SM, pts, bn
-template <class R> GMT_HD void hside_star_adj(const HSide<R>& s, R SM, R pts, R bn, HSideB<R>& b, R& SM_b, R& pts_b,
-                                              R& bn_b) {
-    const R den = s.S - SM;
-    const R num_b = b.Es / den;
-    const R den_b = -b.Es * s.Es / den;
-    b.S += den_b + num_b * s.E;
-    SM_b += -den_b + num_b * pts;
-    b.u += -num_b * s.E - num_b * s.pt;
-    b.E += num_b * (s.S - s.u);
-    b.pt += -num_b * s.u;
-    pts_b += num_b * SM;
-    bn_b += num_b * (s.vdotb - s.vdotbs);
-    const R vdotb_b = num_b * bn;
-    const R vdotbs_b = b.vdotbs - num_b * bn;
-    SM_b += vdotbs_b * bn;
-    bn_b += vdotbs_b * SM;
-    b.vys += vdotbs_b * s.bys; b.bys += vdotbs_b * s.vys;
-    b.vzs += vdotbs_b * s.bzs; b.bzs += vdotbs_b * s.vzs;
-    b.u += vdotb_b * bn; bn_b += vdotb_b * s.u;
-    b.v += vdotb_b * s.by; b.by += vdotb_b * s.v;
-    b.w += vdotb_b * s.bz; b.bz += vdotb_b * s.w;
-    hlld_star_adj(s.d, s.u, s.v, s.w, s.by, s.bz, s.S, SM, bn, b.vys, b.vzs, b.bys, b.bzs, b.d, b.u, b.v, b.w, b.by,
-                  b.bz, b.S, SM_b, bn_b);
-}
-
-// adjoint of U = {d, d u, d v, d w, E, bn, by, bz, 0} (the side's conserved state) for ub
-template <class R> GMT_HD void hside_u_adj(const HSide<R>& s, const R* ub, HSideB<R>& b, R& bn_b) {
-    b.d += ub[0] + ub[1] * s.u + ub[2] * s.v + ub[3] * s.w;
-    b.u += ub[1] * s.d; b.v += ub[2] * s.d; b.w += ub[3] * s.d;
-    b.E += ub[4]; bn_b += ub[5]; b.by += ub[6]; b.bz += ub[7];
-}
-
-// outer region of the HLLD fan on side s: F = F_s + S_s (U*_s - U_s)
-template <class R>
-GMT_HD void hlld_outer_adj(HSide<R>& s, HSideB<R>& b, R ds, R SM, R pts, R bn, const R* g, Q9<R>& Fb, R& ds_b,
-                           R& SM_b, R& pts_b, R& bn_b) {
-    hside_star(s, SM, pts, bn);
-    const R Us[9] = {ds, ds * SM, ds * s.vys, ds * s.vzs, s.Es, bn, s.bys, s.bzs, R(0)};
-    const R U[9] = {s.d, s.d * s.u, s.d * s.v, s.d * s.w, s.E, bn, s.by, s.bz, R(0)};
-    R Usb[9], Ub[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        b.S += g[i] * (Us[i] - U[i]);
-        Usb[i] = g[i] * s.S;
-        Ub[i] = -g[i] * s.S;
-        Fb.v[i] = g[i];
-    }
-    ds_b += Usb[0] + Usb[1] * SM + Usb[2] * s.vys + Usb[3] * s.vzs;
-    SM_b += Usb[1] * ds;
-    b.vys += Usb[2] * ds;
-    b.vzs += Usb[3] * ds;
-    b.Es += Usb[4];
-    bn_b += Usb[5];
-    b.bys += Usb[6];
-    b.bzs += Usb[7];
-    hside_u_adj(s, Ub, b, bn_b);
-    hside_star_adj(s, SM, pts, bn, b, SM_b, pts_b, bn_b);
-}
-
-// inner region: F = F_s + S*s Uss - (S*s - S_s) Us - S_s U on the sampled side s (LO: the left
-// side, SM >= 0; else the right side); both star states are already evaluated
-template <bool LO, class R>
-GMT_HD void hlld_inner_adj(const HSide<R>& sl, const HSide<R>& sr, HSideB<R>& bl, HSideB<R>& br, R ds, R sqdLs,
-                           R sqdRs, R Ssx, R SM, R pts, R bn, const R* g, Q9<R>& Fb, R& ds_b, R& sqdLs_b, R& sqdRs_b,
-                           R& Ssx_b, R& SM_b, R& bn_b) {
-    const HSide<R>& s = LO ? sl : sr;
-    HSideB<R>& b = LO ? bl : br;
-    const R sgn = bn >= R(0) ? R(1) : R(-1);
-    const R ssum = sqdLs + sqdRs;
-    const R invsum = R(1) / ssum;
-    const R nvy = sqdLs * sl.vys + sqdRs * sr.vys + (sr.bys - sl.bys) * sgn;
-    const R nvz = sqdLs * sl.vzs + sqdRs * sr.vzs + (sr.bzs - sl.bzs) * sgn;
-    const R nby = sqdLs * sr.bys + sqdRs * sl.bys + sqdLs * sqdRs * (sr.vys - sl.vys) * sgn;
-    const R nbz = sqdLs * sr.bzs + sqdRs * sl.bzs + sqdLs * sqdRs * (sr.vzs - sl.vzs) * sgn;
-    const R vyss = nvy * invsum, vzss = nvz * invsum, byss = nby * invsum, bzss = nbz * invsum;
-    const R vdotbss = SM * bn + vyss * byss + vzss * bzss;
-    const R sq = LO ? sqdLs : sqdRs;
-    const R sign_e = LO ? R(-1) : R(1);   // ELss = ELs - sq(.)sgn, ERss = ERs + sq(.)sgn
-    const R Ess = s.Es + sign_e * (sq * (s.vdotbs - vdotbss) * sgn);
-    const R Uss[9] = {ds, ds * SM, ds * vyss, ds * vzss, Ess, bn, byss, bzss, R(0)};
-    const R Us[9] = {ds, ds * SM, ds * s.vys, ds * s.vzs, s.Es, bn, s.bys, s.bzs, R(0)};
-    const R U[9] = {s.d, s.d * s.u, s.d * s.v, s.d * s.w, s.E, bn, s.by, s.bz, R(0)};
-    R Ussb[9], Usb[9], Ub[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        Ssx_b += g[i] * (Uss[i] - Us[i]);
-        b.S += g[i] * (Us[i] - U[i]);
-        Ussb[i] = g[i] * Ssx;
-        Usb[i] = -g[i] * (Ssx - s.S);
-        Ub[i] = -g[i] * s.S;
-        Fb.v[i] = g[i];
-    }
-    // Uss
-    ds_b += Ussb[0] + Ussb[1] * SM + Ussb[2] * vyss + Ussb[3] * vzss;
-    SM_b += Ussb[1] * ds;
-    R vyss_b = Ussb[2] * ds, vzss_b = Ussb[3] * ds;
-    const R Ess_b = Ussb[4];
-    bn_b += Ussb[5];
-    R byss_b = Ussb[6], bzss_b = Ussb[7];
-    // Ess = Es + sign_e * sq * (vdotbs - vdotbss) * sgn
-    b.Es += Ess_b;
-    (LO ? sqdLs_b : sqdRs_b) += Ess_b * sign_e * (s.vdotbs - vdotbss) * sgn;
-    b.vdotbs += Ess_b * sign_e * sq * sgn;
-    const R vdotbss_b = -Ess_b * sign_e * sq * sgn;
-    // vdotbss = SM bn + vyss byss + vzss bzss
-    SM_b += vdotbss_b * bn;
-    bn_b += vdotbss_b * SM;
-    vyss_b += vdotbss_b * byss; byss_b += vdotbss_b * vyss;
-    vzss_b += vdotbss_b * bzss; bzss_b += vdotbss_b * vzss;
-    // Us (the sampled side's star state) and U
-    ds_b += Usb[0] + Usb[1] * SM + Usb[2] * s.vys + Usb[3] * s.vzs;
-    SM_b += Usb[1] * ds;
-    b.vys += Usb[2] * ds;
-    b.vzs += Usb[3] * ds;
-    b.Es += Usb[4];
-    bn_b += Usb[5];
-    b.bys += Usb[6];
-    b.bzs += Usb[7];
-    hside_u_adj(s, Ub, b, bn_b);
-    // the double-star averages
-    const R invsum_b = vyss_b * nvy + vzss_b * nvz + byss_b * nby + bzss_b * nbz;
-    const R tvy = vyss_b * invsum, tvz = vzss_b * invsum, tby = byss_b * invsum, tbz = bzss_b * invsum;
-    sqdLs_b += tvy * sl.vys + tvz * sl.vzs + tby * sr.bys + tbz * sr.bzs + tby * sqdRs * (sr.vys - sl.vys) * sgn +
-               tbz * sqdRs * (sr.vzs - sl.vzs) * sgn;
-    sqdRs_b += tvy * sr.vys + tvz * sr.vzs + tby * sl.bys + tbz * sl.bzs + tby * sqdLs * (sr.vys - sl.vys) * sgn +
-               tbz * sqdLs * (sr.vzs - sl.vzs) * sgn;
-    bl.vys += tvy * sqdLs - tby * sqdLs * sqdRs * sgn;
-    br.vys += tvy * sqdRs + tby * sqdLs * sqdRs * sgn;
-    bl.vzs += tvz * sqdLs - tbz * sqdLs * sqdRs * sgn;
-    br.vzs += tvz * sqdRs + tbz * sqdLs * sqdRs * sgn;
-    bl.bys += -tvy * sgn + tby * sqdRs;
-    br.bys += tvy * sgn + tby * sqdLs;
-    bl.bzs += -tvz * sgn + tbz * sqdRs;
-    br.bzs += tvz * sgn + tbz * sqdLs;
-    const R ssum_b = -invsum_b * invsum * invsum;
-    sqdLs_b += ssum_b;
-    sqdRs_b += ssum_b;
-}
-
-// HLLD (hlld_x): Lb, Rb, bnb += adjoint for flux adjoint fb (fb[5], fb[8] do not enter)
+// HLLD (hlld_x): Lb, Rb, bnb += adjoint for flux adjoint fb (fb[5], fb[8] do not enter).
+//
+// The fan is swept in the frame of its sampled side s (the left one when SM >= 0, which every region
+// implies: SL* >= 0 has SM >= 0, SR* < 0 has SM < 0) and the other side o.  SM, pT* and the averages
+// are the same functions of (s, o) as of (L, R): exchanging the sides changes the sign of numerator
+// and denominator alike, and of the double-star differences, which sgn(bn) absorbs.  So one body
+// serves the four regions, F = F_s + S_s (U*_s - U_s), plus S*_s (U**_s - U*_s) in the double-star
+// ones, instead of a copy per region: a warp whose faces lie in different regions no longer runs
+// several of them in turn, and the code fits the instruction cache better (in FP64 the pass spent
+// most of its issue slots waiting for instructions: 64^3 FP64 513 us).  Only s has an energy and a
+// flux of its own in the result, so those of o are not formed, and one fast speed carries the whole
+// adjoint of max(cL, cR).  The branches are decided by the forward step's own expressions; quotients
+// that only enter the adjoint are formed with one reciprocal per divisor.
 template <class R>
 GMT_HD void hlld_x_adj(const Q9<R>& L, const Q9<R>& Rr, R gamma, R bn, const Q9<R>& fb, Q9<R>& Lb, Q9<R>& Rb, R& bnb) {
-    const R tiny = R(1e-12);
-    HSide<R> sl, sr;
-    sl.d = L.v[0]; sl.u = L.v[1]; sl.v = L.v[2]; sl.w = L.v[3]; sl.p = L.v[4]; sl.by = L.v[6]; sl.bz = L.v[7];
-    sr.d = Rr.v[0]; sr.u = Rr.v[1]; sr.v = Rr.v[2]; sr.w = Rr.v[3]; sr.p = Rr.v[4]; sr.by = Rr.v[6]; sr.bz = Rr.v[7];
-    const R b2L = bn * bn + sl.by * sl.by + sl.bz * sl.bz;
-    const R b2R = bn * bn + sr.by * sr.by + sr.bz * sr.bz;
-    sl.pt = sl.p + R(0.5) * b2L;
-    sr.pt = sr.p + R(0.5) * b2R;
-    sl.E = sl.p / (gamma - R(1)) + R(0.5) * sl.d * (sl.u * sl.u + sl.v * sl.v + sl.w * sl.w) + R(0.5) * b2L;
-    sr.E = sr.p / (gamma - R(1)) + R(0.5) * sr.d * (sr.u * sr.u + sr.v * sr.v + sr.w * sr.w) + R(0.5) * b2R;
-    const R cfL = fast_speed(L, gamma, bn), cfR = fast_speed(Rr, gamma, bn);
-    const R umin = rmin(sl.u, sr.u), umax = rmax(sl.u, sr.u), cmax = rmax(cfL, cfR);
-    const R xL = umin - cmax, xR = umax + cmax;
-    sl.S = rmin(xL, R(0));
-    sr.S = rmax(xR, R(0));
-    const R aL = sl.S - sl.u, aR = sr.S - sr.u;
-    const R den = aR * sr.d - aL * sl.d;
-    const R SM = (aR * sr.d * sr.u - aL * sl.d * sl.u - sr.pt + sl.pt) / den;
-    const R du = sr.u - sl.u;
-    const R pts = (aR * sr.d * sl.pt - aL * sl.d * sr.pt + sl.d * sr.d * aR * aL * du) / den;
-    const R qL = sl.d * aL / (sl.S - SM), qR = sr.d * aR / (sr.S - SM);
-    const R dLs = rmax(qL, tiny), dRs = rmax(qR, tiny);
-    const R sqdLs = sqrt_r(dLs), sqdRs = sqrt_r(dRs);
+    const R tiny = R(1e-12), igm1 = R(1) / (gamma - R(1));
+    bool left;
+    R S, oS, SM, pts, cfL, cfR, xL, xR;
+    {
+        const R dL = L.v[0], uL = L.v[1], dR = Rr.v[0], uR = Rr.v[1];
+        const R ptL = L.v[4] + R(0.5) * (bn * bn + L.v[6] * L.v[6] + L.v[7] * L.v[7]);
+        const R ptR = Rr.v[4] + R(0.5) * (bn * bn + Rr.v[6] * Rr.v[6] + Rr.v[7] * Rr.v[7]);
+        cfL = fast_speed(L, gamma, bn);
+        cfR = fast_speed(Rr, gamma, bn);
+        xL = rmin(uL, uR) - rmax(cfL, cfR);
+        xR = rmax(uL, uR) + rmax(cfL, cfR);
+        const R SL = rmin(xL, R(0)), SR = rmax(xR, R(0));
+        const R aL = SL - uL, aR = SR - uR;
+        const R den = aR * dR - aL * dL;
+        SM = (aR * dR * uR - aL * dL * uL - ptR + ptL) / den;
+        pts = (aR * dR * ptL - aL * dL * ptR + dL * dR * aR * aL * (uR - uL)) / den;
+        left = SM >= R(0);
+        S = left ? SL : SR;
+        oS = left ? SR : SL;
+    }
+    const R sig = left ? R(1) : R(-1);
+    // (value by value: a reference chosen at run time would put the states in local memory)
+    const R d = left ? L.v[0] : Rr.v[0], u = left ? L.v[1] : Rr.v[1], v = left ? L.v[2] : Rr.v[2];
+    const R w = left ? L.v[3] : Rr.v[3], p = left ? L.v[4] : Rr.v[4];
+    const R by = left ? L.v[6] : Rr.v[6], bz = left ? L.v[7] : Rr.v[7];
+    const R od = left ? Rr.v[0] : L.v[0], ou = left ? Rr.v[1] : L.v[1], ov = left ? Rr.v[2] : L.v[2];
+    const R ow = left ? Rr.v[3] : L.v[3], op = left ? Rr.v[4] : L.v[4];
+    const R oby = left ? Rr.v[6] : L.v[6], obz = left ? Rr.v[7] : L.v[7];
+    const R b2 = bn * bn + by * by + bz * bz, pt = p + R(0.5) * b2;
+    const R vsq = u * u + v * v + w * w, E = p * igm1 + R(0.5) * d * vsq + R(0.5) * b2;
+    const R opt = op + R(0.5) * (bn * bn + oby * oby + obz * obz);
+    const R a = S - u, oa = oS - ou, l = S - SM, ol = oS - SM;
+    const R il = R(1) / l;
+    const R q = d * a / l, oq = od * oa / ol;
+    const R ds = rmax(q, tiny), ods = rmax(oq, tiny);
+    const R sq = sqrt_r(ds), osq = sqrt_r(ods);
     const R abn = rabs(bn);
-    const R SLs = SM - abn / sqdLs;
-    const R SRs = SM + abn / sqdRs;
+    const R Ss = SM - sig * (abn / sq);                       // S*_L or S*_R
+    const bool inner = left ? Ss < R(0) : Ss >= R(0);
 
-    R g[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) g[i] = (i == 5 || i == 8) ? R(0) : fb.v[i];
-    HSideB<R> bl, br;
-    hside_zero(bl);
-    hside_zero(br);
-    R SM_b = R(0), pts_b = R(0), bn_b = R(0), SLs_b = R(0), SRs_b = R(0), dLs_b = R(0), dRs_b = R(0);
-    R sqdLs_b = R(0), sqdRs_b = R(0);
-    Q9<R> FLb, FRb;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) { FLb.v[i] = R(0); FRb.v[i] = R(0); }
-    if (SLs >= R(0)) {
-        hlld_outer_adj(sl, bl, dLs, SM, pts, bn, g, FLb, dLs_b, SM_b, pts_b, bn_b);
-    } else if (SRs < R(0)) {
-        hlld_outer_adj(sr, br, dRs, SM, pts, bn, g, FRb, dRs_b, SM_b, pts_b, bn_b);
-    } else {
-        hside_star(sl, SM, pts, bn);
-        hside_star(sr, SM, pts, bn);
-        if (SM >= R(0))
-            hlld_inner_adj<true>(sl, sr, bl, br, dLs, sqdLs, sqdRs, SLs, SM, pts, bn, g, FLb, dLs_b, sqdLs_b, sqdRs_b,
-                                 SLs_b, SM_b, bn_b);
-        else
-            hlld_inner_adj<false>(sl, sr, bl, br, dRs, sqdLs, sqdRs, SRs, SM, pts, bn, g, FRb, dRs_b, sqdLs_b, sqdRs_b,
-                                  SRs_b, SM_b, bn_b);
-        hside_star_adj(sl, SM, pts, bn, bl, SM_b, pts_b, bn_b);
-        hside_star_adj(sr, SM, pts, bn, br, SM_b, pts_b, bn_b);
+    // forward: the star state of s
+    const HStar<R> st = hstar(d, u, v, w, by, bz, S, SM, bn);
+    const R vdotb = u * bn + v * by + w * bz, vdotbs = SM * bn + st.vy * st.by + st.vz * st.bz;
+    const R Es = (a * E - pt * u + pts * SM + bn * (vdotb - vdotbs)) * il;
+
+    const R g0 = fb.v[0], g1 = fb.v[1], g2 = fb.v[2], g3 = fb.v[3], g4 = fb.v[4], g6 = fb.v[6], g7 = fb.v[7];
+    // F_s + S (U* - U): adjoints of U* (gs), of U (-S g) and of S
+    R SM_b = g1 * S * ds, bn_b = R(0);
+    R S_b = g0 * (ds - d) + g1 * (ds * SM - d * u) + g2 * (ds * st.vy - d * v) + g3 * (ds * st.vz - d * w) +
+            g4 * (Es - E) + g6 * (st.by - by) + g7 * (st.bz - bz);
+    R f = S;                                                    // U*'s weight: S, less S* in the double star
+    R sq_b = R(0), osq_b = R(0), Ss_b = R(0), oS_b = R(0);
+    R vy_b = R(0), vz_b = R(0), bys_b = R(0), bzs_b = R(0), vdotbs_b = R(0), Es_b = R(0), ds_b = R(0);
+    R d_b = R(0), u_b = R(0), v_b = R(0), w_b = R(0), by_b = R(0), bz_b = R(0), E_b, pt_b;
+    R od_b = R(0), ou_b = R(0), ov_b = R(0), ow_b = R(0), oby_b = R(0), obz_b = R(0), opt_b;
+    if (inner) {
+        const HStar<R> ot = hstar(od, ou, ov, ow, oby, obz, oS, SM, bn);
+        const R sg = bn >= R(0) ? sig : -sig, invsum = R(1) / (sq + osq), sqq = sq * osq;
+        const R vyss = (sq * st.vy + osq * ot.vy + (ot.by - st.by) * sg) * invsum;
+        const R vzss = (sq * st.vz + osq * ot.vz + (ot.bz - st.bz) * sg) * invsum;
+        const R byss = (sq * ot.by + osq * st.by + sqq * (ot.vy - st.vy) * sg) * invsum;
+        const R bzss = (sq * ot.bz + osq * st.bz + sqq * (ot.vz - st.vz) * sg) * invsum;
+        const R vdotbss = SM * bn + vyss * byss + vzss * bzss;
+        const R dv = vdotbs - vdotbss;
+        // F += S* (U** - U*), U**'s energy Es - sq (v.B* - v.B**) sgn
+        Ss_b = g2 * ds * (vyss - st.vy) + g3 * ds * (vzss - st.vz) - g4 * sq * dv * sg + g6 * (byss - st.by) +
+               g7 * (bzss - st.bz);
+        f = S - Ss;
+        const R e = g4 * Ss * sg;
+        sq_b = -e * dv;
+        vdotbs_b = -e * sq;
+        const R vdotbss_b = e * sq;
+        ds_b = Ss * (g0 + g1 * SM + g2 * vyss + g3 * vzss);
+        SM_b += g1 * Ss * ds + vdotbss_b * bn;
+        bn_b += vdotbss_b * SM;
+        Es_b = g4 * Ss;
+        // the averages (divided by the sum of roots)
+        const R tvy = (g2 * Ss * ds + vdotbss_b * byss) * invsum, tvz = (g3 * Ss * ds + vdotbss_b * bzss) * invsum;
+        const R tby = (g6 * Ss + vdotbss_b * vyss) * invsum, tbz = (g7 * Ss + vdotbss_b * vzss) * invsum;
+        const R sum_b = -(tvy * vyss + tvz * vzss + tby * byss + tbz * bzss);
+        const R cross = (tby * (ot.vy - st.vy) + tbz * (ot.vz - st.vz)) * sg;
+        sq_b += tvy * st.vy + tvz * st.vz + tby * ot.by + tbz * ot.bz + osq * cross + sum_b;
+        osq_b = tvy * ot.vy + tvz * ot.vz + tby * st.by + tbz * st.bz + sq * cross + sum_b;
+        vy_b = tvy * sq - tby * sqq * sg;
+        vz_b = tvz * sq - tbz * sqq * sg;
+        bys_b = -tvy * sg + tby * osq;
+        bzs_b = -tvz * sg + tbz * osq;
+        hstar_adj(od, ou, oby, obz, oS, SM, bn, ot, tvy * osq + tby * sqq * sg, tvz * osq + tbz * sqq * sg,
+                  tvy * sg + tby * sq, tvz * sg + tbz * sq, od_b, ou_b, ov_b, ow_b, oby_b, obz_b, oS_b, SM_b, bn_b);
+        // S* = SM - sig |bn| / sq
+        const R isq = R(1) / sq, h = sig * Ss_b * isq;
+        SM_b += Ss_b;
+        bn_b += bn >= R(0) ? -h : h;
+        sq_b += h * abn * isq;
     }
-    // SLs = SM - |bn| / sqdLs, SRs = SM + |bn| / sqdRs
-    SM_b += SLs_b + SRs_b;
-    const R abn_b = -SLs_b / sqdLs + SRs_b / sqdRs;
-    sqdLs_b += SLs_b * abn / (sqdLs * sqdLs);
-    sqdRs_b += -SRs_b * abn / (sqdRs * sqdRs);
-    bn_b += abn_b * (bn >= R(0) ? R(1) : R(-1));
-    // sqrt and the tiny floors
-    dLs_b += sqdLs > R(0) ? sqdLs_b * (R(0.5) / sqdLs) : R(0);
-    dRs_b += sqdRs > R(0) ? sqdRs_b * (R(0.5) / sqdRs) : R(0);
-    const R qL_b = dLs_b * sel_ge(qL, tiny), qR_b = dRs_b * sel_ge(qR, tiny);
-    {
-        const R dl = sl.S - SM, num_b = qL_b / dl, dl_b = -qL_b * qL / dl;
-        bl.d += num_b * aL;
-        R aL_b = num_b * sl.d;
-        bl.S += dl_b;
-        SM_b -= dl_b;
-        const R dr = sr.S - SM, numr_b = qR_b / dr, dr_b = -qR_b * qR / dr;
-        br.d += numr_b * aR;
-        R aR_b = numr_b * sr.d;
-        br.S += dr_b;
-        SM_b -= dr_b;
-        // pts = (aR dR ptL - aL dL ptR + dL dR aR aL du) / den ; SM = (aR dR uR - aL dL uL - ptR + ptL) / den
-        const R ptsn_b = pts_b / den;
-        R den_b = -pts_b * pts / den;
-        const R smn_b = SM_b / den;
-        den_b += -SM_b * SM / den;
-        aR_b += ptsn_b * sr.d * sl.pt + ptsn_b * sl.d * sr.d * aL * du + smn_b * sr.d * sr.u + den_b * sr.d;
-        aL_b += -ptsn_b * sl.d * sr.pt + ptsn_b * sl.d * sr.d * aR * du - smn_b * sl.d * sl.u - den_b * sl.d;
-        br.d += ptsn_b * aR * sl.pt + ptsn_b * sl.d * aR * aL * du + smn_b * aR * sr.u + den_b * aR;
-        bl.d += -ptsn_b * aL * sr.pt + ptsn_b * sr.d * aR * aL * du - smn_b * aL * sl.u - den_b * aL;
-        bl.pt += ptsn_b * aR * sr.d + smn_b;
-        br.pt += -ptsn_b * aL * sl.d - smn_b;
-        const R du_b = ptsn_b * sl.d * sr.d * aR * aL;
-        br.u += du_b + smn_b * aR * sr.d - aR_b;
-        bl.u += -du_b - smn_b * aL * sl.d - aL_b;
-        bl.S += aL_b;
-        br.S += aR_b;
+    // U* = (ds, ds SM, ds vy*, ds vz*, Es, bn, by*, bz*) with weight f; U with weight -S
+    ds_b += f * (g0 + g1 * SM + g2 * st.vy + g3 * st.vz);
+    if (inner) SM_b -= g1 * Ss * ds;                            // (f - S) g1 ds
+    vy_b += f * g2 * ds;
+    vz_b += f * g3 * ds;
+    bys_b += f * g6;
+    bzs_b += f * g7;
+    Es_b += f * g4;
+    d_b -= S * (g0 + g1 * u + g2 * v + g3 * w);
+    u_b -= S * g1 * d; v_b -= S * g2 * d; w_b -= S * g3 * d;
+    E_b = -S * g4;
+    by_b -= S * g6; bz_b -= S * g7;
+    // Es = (a E - pt u + pts SM + bn (v.B - v.B*)) / l
+    const R n_b = Es_b * il, l_b0 = -n_b * Es;
+    R pts_b = n_b * SM;
+    S_b += l_b0 + n_b * E;
+    SM_b += n_b * pts - l_b0;
+    u_b -= n_b * (E + pt);
+    E_b += n_b * a;
+    pt_b = -n_b * u;
+    const R vdotb_b = n_b * bn;
+    vdotbs_b -= vdotb_b;
+    bn_b += n_b * (vdotb - vdotbs) + vdotbs_b * SM + vdotb_b * u;
+    SM_b += vdotbs_b * bn;
+    vy_b += vdotbs_b * st.by; bys_b += vdotbs_b * st.vy;
+    vz_b += vdotbs_b * st.bz; bzs_b += vdotbs_b * st.vz;
+    u_b += vdotb_b * bn;
+    v_b += vdotb_b * by; by_b += vdotb_b * v;
+    w_b += vdotb_b * bz; bz_b += vdotb_b * w;
+    hstar_adj(d, u, by, bz, S, SM, bn, st, vy_b, vz_b, bys_b, bzs_b, d_b, u_b, v_b, w_b, by_b, bz_b, S_b, SM_b, bn_b);
+    // roots and floors, then rho* = d a / l of either side
+    ds_b += sq > R(0) ? sq_b * (R(0.5) / sq) : R(0);
+    const R q_b = ds_b * sel_ge(q, tiny) * il;
+    R a_b = q_b * d;
+    d_b += q_b * a;
+    S_b -= q_b * q;
+    SM_b += q_b * q;
+    R oa_b = R(0);
+    if (inner) {
+        const R oq_b = (osq > R(0) ? osq_b * (R(0.5) / osq) : R(0)) * sel_ge(oq, tiny) / ol;
+        oa_b = oq_b * od;
+        od_b += oq_b * oa;
+        oS_b -= oq_b * oq;
+        SM_b += oq_b * oq;
     }
-    // S_L = min(min(uL, uR) - max(cfL, cfR), 0), S_R = max(max(uL, uR) + max(cfL, cfR), 0)
-    const R xL_b = bl.S * sel_le(xL, R(0)), xR_b = br.S * sel_ge(xR, R(0));
-    const R umin_b = xL_b, umax_b = xR_b, cmax_b = -xL_b + xR_b;
-    const R ul_min = sel_le(sl.u, sr.u), ul_max = sel_ge(sl.u, sr.u), cl_max = sel_ge(cfL, cfR);
-    bl.u += umin_b * ul_min + umax_b * ul_max;
-    br.u += umin_b * (R(1) - ul_min) + umax_b * (R(1) - ul_max);
-    fast_speed_adj(L, gamma, bn, cmax_b * cl_max, Lb, bn_b);
-    fast_speed_adj(Rr, gamma, bn, cmax_b * (R(1) - cl_max), Rb, bn_b);
-    // the outer-side fluxes F_s = phys_flux_x({d, u, v, w, p, bn, by, bz, 0})
     {
-        Q9<R> qLf, qRf, qLb, qRb;
-#pragma unroll
-        for (int i = 0; i < 9; ++i) { qLb.v[i] = R(0); qRb.v[i] = R(0); }
-        qLf.v[0] = sl.d; qLf.v[1] = sl.u; qLf.v[2] = sl.v; qLf.v[3] = sl.w; qLf.v[4] = sl.p;
-        qLf.v[5] = bn; qLf.v[6] = sl.by; qLf.v[7] = sl.bz; qLf.v[8] = R(0);
-        qRf.v[0] = sr.d; qRf.v[1] = sr.u; qRf.v[2] = sr.v; qRf.v[3] = sr.w; qRf.v[4] = sr.p;
-        qRf.v[5] = bn; qRf.v[6] = sr.by; qRf.v[7] = sr.bz; qRf.v[8] = R(0);
-        phys_flux_x_adj(qLf, gamma, FLb, qLb);
-        phys_flux_x_adj(qRf, gamma, FRb, qRb);
-        bl.d += qLb.v[0]; bl.u += qLb.v[1]; bl.v += qLb.v[2]; bl.w += qLb.v[3]; bl.p += qLb.v[4];
-        bn_b += qLb.v[5] + qRb.v[5];
-        bl.by += qLb.v[6]; bl.bz += qLb.v[7];
-        br.d += qRb.v[0]; br.u += qRb.v[1]; br.v += qRb.v[2]; br.w += qRb.v[3]; br.p += qRb.v[4];
-        br.by += qRb.v[6]; br.bz += qRb.v[7];
+        // pts and SM over den = oa od - a d (with s in the place of L)
+        const R m = a * d, om = oa * od, iden = R(1) / (om - m), du = ou - u;
+        const R tn = pts_b * iden, sn = SM_b * iden, den_b = -(tn * pts + sn * SM);
+        const R om_b = tn * (pt + m * du) + sn * ou + den_b, m_b = tn * (om * du - opt) - sn * u - den_b;
+        oa_b += om_b * od;
+        od_b += om_b * oa;
+        a_b += m_b * d;
+        d_b += m_b * a;
+        pt_b += tn * om + sn;
+        opt_b = -tn * m - sn;
+        const R du_b = tn * m * om;
+        ou_b += du_b + sn * om - oa_b;
+        u_b += -du_b - sn * m - a_b;
+        S_b += a_b;
+        oS_b += oa_b;
     }
-    // E_s = p/(gamma-1) + d|v|^2/2 + b2/2, pt_s = p + b2/2, b2_s = bn^2 + by^2 + bz^2
+    // F_s = phys_flux_x of (d, u, v, w, p, bn, by, bz)
+    R p_b = R(0);
     {
-        HSide<R>* ss[2] = {&sl, &sr};
-        HSideB<R>* bb[2] = {&bl, &br};
-        Q9<R>* out[2] = {&Lb, &Rb};
+        const Q9<R> qf{{d, u, v, w, p, bn, by, bz, R(0)}};
+        const Q9<R> gf{{g0, g1, g2, g3, g4, R(0), g6, g7, R(0)}};
+        Q9<R> qb;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const HSide<R>& s = *ss[k];
-            HSideB<R>& b = *bb[k];
-            const R b2_b = R(0.5) * b.E + R(0.5) * b.pt;
-            b.p += b.E / (gamma - R(1)) + b.pt;
-            b.d += b.E * R(0.5) * (s.u * s.u + s.v * s.v + s.w * s.w);
-            b.u += b.E * s.d * s.u;
-            b.v += b.E * s.d * s.v;
-            b.w += b.E * s.d * s.w;
-            bn_b += b2_b * R(2) * bn;
-            b.by += b2_b * R(2) * s.by;
-            b.bz += b2_b * R(2) * s.bz;
-            Q9<R>& o = *out[k];
-            o.v[0] += b.d; o.v[1] += b.u; o.v[2] += b.v; o.v[3] += b.w; o.v[4] += b.p;
-            o.v[6] += b.by; o.v[7] += b.bz;
+        for (int i = 0; i < 9; ++i) qb.v[i] = R(0);
+        phys_flux_x_adj(qf, gamma, gf, qb);
+        d_b += qb.v[0]; u_b += qb.v[1]; v_b += qb.v[2]; w_b += qb.v[3]; p_b += qb.v[4];
+        bn_b += qb.v[5]; by_b += qb.v[6]; bz_b += qb.v[7];
+    }
+    // E = p/(gamma-1) + d|v|^2/2 + b2/2, pt = p + b2/2 (of o only pt)
+    const R b2_b = E_b + pt_b;                                  // twice the adjoint of b2
+    p_b += E_b * igm1 + pt_b;
+    d_b += E_b * R(0.5) * vsq;
+    u_b += E_b * d * u; v_b += E_b * d * v; w_b += E_b * d * w;
+    by_b += b2_b * by; bz_b += b2_b * bz;
+    oby_b += opt_b * oby; obz_b += opt_b * obz;
+    bn_b += (b2_b + opt_b) * bn;
+    // back to L and R
+    const R SL_b = left ? S_b : oS_b, SR_b = left ? oS_b : S_b;
+    const R xL_b = SL_b * sel_le(xL, R(0)), xR_b = SR_b * sel_ge(xR, R(0));
+    const R ul_min = sel_le(L.v[1], Rr.v[1]), ul_max = sel_ge(L.v[1], Rr.v[1]);
+    const R uLx = xL_b * ul_min + xR_b * ul_max, uRx = xL_b + xR_b - uLx;
+    Lb.v[0] += left ? d_b : od_b;   Rb.v[0] += left ? od_b : d_b;
+    Lb.v[1] += (left ? u_b : ou_b) + uLx;
+    Rb.v[1] += (left ? ou_b : u_b) + uRx;
+    Lb.v[2] += left ? v_b : ov_b;   Rb.v[2] += left ? ov_b : v_b;
+    Lb.v[3] += left ? w_b : ow_b;   Rb.v[3] += left ? ow_b : w_b;
+    Lb.v[4] += left ? p_b : opt_b;  Rb.v[4] += left ? opt_b : p_b;
+    Lb.v[6] += left ? by_b : oby_b; Rb.v[6] += left ? oby_b : by_b;
+    Lb.v[7] += left ? bz_b : obz_b; Rb.v[7] += left ? obz_b : bz_b;
+    // max(cL, cR) takes the side of the larger speed
+    {
+        const bool cl = cfL >= cfR;
+        Q9<R> c, cb;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            c.v[i] = cl ? L.v[i] : Rr.v[i];
+            cb.v[i] = R(0);
         }
+        fast_speed_adj(c, gamma, bn, xR_b - xL_b, cb, bn_b);
+        const R m = cl ? R(1) : R(0), om = R(1) - m;
+        Lb.v[0] += cb.v[0] * m; Rb.v[0] += cb.v[0] * om;
+        Lb.v[4] += cb.v[4] * m; Rb.v[4] += cb.v[4] * om;
+        Lb.v[5] += cb.v[5] * m; Rb.v[5] += cb.v[5] * om;
+        Lb.v[6] += cb.v[6] * m; Rb.v[6] += cb.v[6] * om;
+        Lb.v[7] += cb.v[7] * m; Rb.v[7] += cb.v[7] * om;
     }
     bnb += bn_b;
 }
