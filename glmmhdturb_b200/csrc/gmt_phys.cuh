@@ -495,71 +495,51 @@ template <class R> GMT_HD Q9<R> hlld_x(const Q9<R>& L, const Q9<R>& Rr, R gamma,
     R den = (SR - uR) * dR - (SL - uL) * dL;
     R SM = ((SR - uR) * dR * uR - (SL - uL) * dL * uL - ptR + ptL) / den;
     R pts = ((SR - uR) * dR * ptL - (SL - uL) * dL * ptR + dL * dR * (SR - uR) * (SL - uL) * (uR - uL)) / den;
-    R dLs = rmax(dL * (SL - uL) / (SL - SM), tiny);
-    R dRs = rmax(dR * (SR - uR) / (SR - SM), tiny);
-    R sqdLs = sqrt_r(dLs), sqdRs = sqrt_r(dRs);
-    R SLs = SM - rabs(bn) / sqdLs;
-    R SRs = SM + rabs(bn) / sqdRs;
+    // The sampled side s: the left one when SM >= 0, which every region implies (SL* >= 0 has SM >= 0,
+    // SR* < 0 has SM < 0).  The four regions are F_s + S (U* - U) and, in the double star,
+    // F_s + S* U** - (S* - S) U* - S U, in either frame by the same operations: sums commute, and a
+    // sign carried by sig or sg is exact, so both frames round alike.  One body instead of four keeps a
+    // warp whose faces lie in different regions from running them in turn (192^3 FP64 step: see
+    // gmt_passes.cuh) and the code in the instruction cache.
+    const bool left = SM >= R(0);
+    const R sig = left ? R(1) : R(-1);
+    const R d = left ? dL : dR, u = left ? uL : uR, v = left ? vL : vR, w = left ? wL : wR, p = left ? pL : pR;
+    const R by = left ? byL : byR, bz = left ? bzL : bzR, pt = left ? ptL : ptR, E = left ? EL : ER;
+    const R S = left ? SL : SR;
+    const R ds = rmax(d * (S - u) / (S - SM), tiny);
+    const R sq = sqrt_r(ds);
+    const R Ss = SM - sig * (rabs(bn) / sq);
+    R vys, vzs, bys, bzs;
+    hlld_star(d, u, v, w, by, bz, S, SM, bn, vys, vzs, bys, bzs);
+    const R vdotb = u * bn + v * by + w * bz;
+    const R vdotbs = SM * bn + vys * bys + vzs * bzs;
+    const R Es = ((S - u) * E - pt * u + pts * SM + bn * (vdotb - vdotbs)) / (S - SM);
+    const Q9<R> Fs = phys_flux_x(Q9<R>{{d, u, v, w, p, bn, by, bz, R(0)}}, gamma);
+    const R Us[9] = {ds, ds * SM, ds * vys, ds * vzs, Es, bn, bys, bzs, R(0)};
+    const R U[9] = {d, d * u, d * v, d * w, E, bn, by, bz, R(0)};
     Q9<R> f;
-    // The flux of the sampled region only needs the states on its side of the fan.
-    if (SLs >= R(0)) {
-        // F = FL + SL*(UL* - UL)
-        R vyLs, vzLs, byLs, bzLs;
-        hlld_star(dL, uL, vL, wL, byL, bzL, SL, SM, bn, vyLs, vzLs, byLs, bzLs);
-        R vdotbL = uL * bn + vL * byL + wL * bzL;
-        R vdotbLs = SM * bn + vyLs * byLs + vzLs * bzLs;
-        R ELs = ((SL - uL) * EL - ptL * uL + pts * SM + bn * (vdotbL - vdotbLs)) / (SL - SM);
-        Q9<R> FL = phys_flux_x(Q9<R>{{dL, uL, vL, wL, pL, bn, byL, bzL, R(0)}}, gamma);
-        R ULs[9] = {dLs, dLs * SM, dLs * vyLs, dLs * vzLs, ELs, bn, byLs, bzLs, R(0)};
-        R UL[9] = {dL, dL * uL, dL * vL, dL * wL, EL, bn, byL, bzL, R(0)};
+    if (left ? Ss >= R(0) : Ss < R(0)) {
 #pragma unroll
-        for (int i = 0; i < 9; ++i) f.v[i] = FL.v[i] + SL * (ULs[i] - UL[i]);
-    } else if (SRs < R(0)) {
-        R vyRs, vzRs, byRs, bzRs;
-        hlld_star(dR, uR, vR, wR, byR, bzR, SR, SM, bn, vyRs, vzRs, byRs, bzRs);
-        R vdotbR = uR * bn + vR * byR + wR * bzR;
-        R vdotbRs = SM * bn + vyRs * byRs + vzRs * bzRs;
-        R ERs = ((SR - uR) * ER - ptR * uR + pts * SM + bn * (vdotbR - vdotbRs)) / (SR - SM);
-        Q9<R> FR = phys_flux_x(Q9<R>{{dR, uR, vR, wR, pR, bn, byR, bzR, R(0)}}, gamma);
-        R URs[9] = {dRs, dRs * SM, dRs * vyRs, dRs * vzRs, ERs, bn, byRs, bzRs, R(0)};
-        R UR[9] = {dR, dR * uR, dR * vR, dR * wR, ER, bn, byR, bzR, R(0)};
-#pragma unroll
-        for (int i = 0; i < 9; ++i) f.v[i] = FR.v[i] + SR * (URs[i] - UR[i]);
+        for (int i = 0; i < 9; ++i) f.v[i] = Fs.v[i] + S * (Us[i] - U[i]);
     } else {
-        // inner fan: both star states and the double-star state
-        R vyLs, vzLs, byLs, bzLs, vyRs, vzRs, byRs, bzRs;
-        hlld_star(dL, uL, vL, wL, byL, bzL, SL, SM, bn, vyLs, vzLs, byLs, bzLs);
-        hlld_star(dR, uR, vR, wR, byR, bzR, SR, SM, bn, vyRs, vzRs, byRs, bzRs);
-        R vdotbL = uL * bn + vL * byL + wL * bzL;
-        R vdotbLs = SM * bn + vyLs * byLs + vzLs * bzLs;
-        R ELs = ((SL - uL) * EL - ptL * uL + pts * SM + bn * (vdotbL - vdotbLs)) / (SL - SM);
-        R vdotbR = uR * bn + vR * byR + wR * bzR;
-        R vdotbRs = SM * bn + vyRs * byRs + vzRs * bzRs;
-        R ERs = ((SR - uR) * ER - ptR * uR + pts * SM + bn * (vdotbR - vdotbRs)) / (SR - SM);
-        R sgn = bn >= R(0) ? R(1) : R(-1);
-        R invsum = R(1) / (sqdLs + sqdRs);
-        R vyss = (sqdLs * vyLs + sqdRs * vyRs + (byRs - byLs) * sgn) * invsum;
-        R vzss = (sqdLs * vzLs + sqdRs * vzRs + (bzRs - bzLs) * sgn) * invsum;
-        R byss = (sqdLs * byRs + sqdRs * byLs + sqdLs * sqdRs * (vyRs - vyLs) * sgn) * invsum;
-        R bzss = (sqdLs * bzRs + sqdRs * bzLs + sqdLs * sqdRs * (vzRs - vzLs) * sgn) * invsum;
-        R vdotbss = SM * bn + vyss * byss + vzss * bzss;
-        if (SM >= R(0)) {
-            R ELss = ELs - sqdLs * (vdotbLs - vdotbss) * sgn;
-            Q9<R> FL = phys_flux_x(Q9<R>{{dL, uL, vL, wL, pL, bn, byL, bzL, R(0)}}, gamma);
-            R ULss[9] = {dLs, dLs * SM, dLs * vyss, dLs * vzss, ELss, bn, byss, bzss, R(0)};
-            R ULs[9] = {dLs, dLs * SM, dLs * vyLs, dLs * vzLs, ELs, bn, byLs, bzLs, R(0)};
-            R UL[9] = {dL, dL * uL, dL * vL, dL * wL, EL, bn, byL, bzL, R(0)};
+        // inner fan: the other side's star state and the double-star averages
+        const R od = left ? dR : dL, ou = left ? uR : uL, oS = left ? SR : SL;
+        const R ods = rmax(od * (oS - ou) / (oS - SM), tiny);
+        const R osq = sqrt_r(ods);
+        R ovy, ovz, oby, obz;
+        hlld_star(od, ou, left ? vR : vL, left ? wR : wL, left ? byR : byL, left ? bzR : bzL, oS, SM, bn, ovy, ovz, oby,
+                  obz);
+        const R sg = bn >= R(0) ? sig : -sig;
+        const R invsum = R(1) / (sq + osq);
+        const R vyss = (sq * vys + osq * ovy + (oby - bys) * sg) * invsum;
+        const R vzss = (sq * vzs + osq * ovz + (obz - bzs) * sg) * invsum;
+        const R byss = (sq * oby + osq * bys + sq * osq * (ovy - vys) * sg) * invsum;
+        const R bzss = (sq * obz + osq * bzs + sq * osq * (ovz - vzs) * sg) * invsum;
+        const R vdotbss = SM * bn + vyss * byss + vzss * bzss;
+        const R Ess = Es - sq * (vdotbs - vdotbss) * sg;
+        const R Uss[9] = {ds, ds * SM, ds * vyss, ds * vzss, Ess, bn, byss, bzss, R(0)};
 #pragma unroll
-            for (int i = 0; i < 9; ++i) f.v[i] = FL.v[i] + SLs * ULss[i] - (SLs - SL) * ULs[i] - SL * UL[i];
-        } else {
-            R ERss = ERs + sqdRs * (vdotbRs - vdotbss) * sgn;
-            Q9<R> FR = phys_flux_x(Q9<R>{{dR, uR, vR, wR, pR, bn, byR, bzR, R(0)}}, gamma);
-            R URss[9] = {dRs, dRs * SM, dRs * vyss, dRs * vzss, ERss, bn, byss, bzss, R(0)};
-            R URs[9] = {dRs, dRs * SM, dRs * vyRs, dRs * vzRs, ERs, bn, byRs, bzRs, R(0)};
-            R UR[9] = {dR, dR * uR, dR * vR, dR * wR, ER, bn, byR, bzR, R(0)};
-#pragma unroll
-            for (int i = 0; i < 9; ++i) f.v[i] = FR.v[i] + SRs * URss[i] - (SRs - SR) * URs[i] - SR * UR[i];
-        }
+        for (int i = 0; i < 9; ++i) f.v[i] = Fs.v[i] + Ss * Uss[i] - (Ss - S) * Us[i] - S * U[i];
     }
     f.v[5] = fbn; f.v[8] = fpsi;
     return f;
