@@ -378,14 +378,6 @@ template <int RIEM, bool DUALS, class R> GMT_HD void adj_riemann_cell(const AdjA
 }
 
 // pass 5: adjoint of the reconstruction of cell c
-// FSbar source reading the scratch planes
-template <class R> struct FaceBarGlobal {
-    const R* FSb;
-    size_t n, c;
-    GMT_HD Q9<R> operator()(int k) const { return fs_get(FSb, n, c, k); }
-    GMT_HD void release() const {}
-};
-
 // the reconstruction adjoint of cell c from its reconstruction r and the adjoints of its six
 // interface states (FB(k), k = +x, -x, +y, -y, +z, -z); FB(k) is called once per face, in face order,
 // and FB.release() once all six have been read
@@ -451,13 +443,168 @@ GMT_HD void adj_recon_core(const AdjArgs<R>& A, size_t n, size_t c, const CellRe
         A.QB[(size_t)v * n + c] = own;
     }
 }
-template <class R> GMT_HD void adj_recon_cell(const AdjArgs<R>& A, size_t c) {
+// ---- passes 1 and 5 from primitive planes (FP64) --------------------------------------------------
+// Q: 9 planes of primitives.  The passes above convert a cell's seven stencil states each time; here
+// that is one pass of its own, and the reconstruction's adjoint goes direction by direction, reloading
+// a direction's two neighbours and two interface-state adjoints where it needs them, instead of
+// carrying all 54 + 54 of them: in FP64 those did not fit the registers (168 at three blocks per SM,
+// 3.2 KB of spill stores per thread, the pass waiting for them: 64^3 207 us).
+template <class R> GMT_HD void adj_prim_cell(const AdjArgs<R>& A, R* Q, size_t c) {
+    const size_t n = (size_t)A.nx * A.ny * A.nz;
+    const Q9<R> q = cons2prim(load_u(A.u, c), A.K.gamma, A.K.smallr, A.K.pfl);
+#pragma unroll
+    for (int v = 0; v < 9; ++v) Q[(size_t)v * n + c] = q.v[v];
+}
+// differences of the prims of cell c to its neighbours cl, cr along an axis, and the half slope
+template <class R>
+GMT_HD void prim_slope(const R* Q, size_t n, const Q9<R>& m0, size_t cl, size_t cr, bool mm, Q9<R>& dl, Q9<R>& dr,
+                       Q9<R>& s) {
+#pragma unroll
+    for (int v = 0; v < 9; ++v) {
+        dl.v[v] = m0.v[v] - Q[(size_t)v * n + cl];
+        dr.v[v] = Q[(size_t)v * n + cr] - m0.v[v];
+        s.v[v] = mm ? R(0.5) * minmod(dl.v[v], dr.v[v]) : R(0.5) * moncen(dl.v[v], dr.v[v]);
+    }
+}
+// the predictor's conserved state: hancock() with the three directions in turn
+template <class R>
+GMT_HD Q9<R> prim_hancock(const R* Q, size_t n, const Q9<R>& m0, const size_t (&cs)[7], R dtdx, R gamma, bool mm) {
+    Q9<R> sum;
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) {
+        Q9<R> dl, dr, sl;
+        const size_t cl = d == 0 ? cs[1] : (d == 1 ? cs[3] : cs[5]), cr = d == 0 ? cs[2] : (d == 1 ? cs[4] : cs[6]);
+        prim_slope(Q, n, m0, cl, cr, mm, dl, dr, sl);
+        const Q9<R> fp = rot_from_d(phys_flux_x(rot_to_d(padd(m0, sl, R(1)), d), gamma), d);
+        const Q9<R> fm = rot_from_d(phys_flux_x(rot_to_d(padd(m0, sl, R(-1)), d), gamma), d);
+#pragma unroll
+        for (int v = 0; v < 9; ++v) sum.v[v] = d == 0 ? fp.v[v] - fm.v[v] : sum.v[v] + (fp.v[v] - fm.v[v]);
+    }
+    const Q9<R> u0 = prim2cons(m0, gamma);
+    const R h = R(0.5) * dtdx;
+    Q9<R> r;
+#pragma unroll
+    for (int v = 0; v < 9; ++v) r.v[v] = u0.v[v] - h * sum.v[v];
+    return r;
+}
+template <class R> GMT_HD void adj_faces_prim_cell(const AdjArgs<R>& A, const R* Q, size_t c) {
     const Idx<R> I = idx_of(A);
+    const bool mm = A.recon == RECON_MINMOD;
     int x, y, z;
     cell_xyz(A, c, x, y, z);
-    CellRec<R> r;
-    cell_rec(A.u, I, x, y, z, A.K, A.dtdx, A.iflo, A.recon == RECON_MINMOD, r);
-    adj_recon_core(A, I.n, c, r, FaceBarGlobal<R>{A.FSb, I.n, c});
+    size_t cs[7];
+    stencil7(I, x, y, z, cs);
+    const Q9<R> m0 = fs_get(Q, I.n, c, 0);
+    Q9<R> mh = cons2prim(prim_hancock(Q, I.n, m0, cs, A.dtdx, A.K.gamma, mm), A.K.gamma, A.K.smallr, A.K.pfl);
+    if (mh.v[0] <= A.K.smallr || mh.v[4] <= A.K.pfl) mh = m0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        Q9<R> dl, dr, sl;
+        prim_slope(Q, I.n, m0, cs[1 + 2 * d], cs[2 + 2 * d], mm, dl, dr, sl);
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            Q9<R> f = padd(mh, sl, side ? R(-1) : R(1));
+            if (A.iflo && (f.v[0] < A.K.smallr || f.v[4] < A.K.pfl)) f = m0;
+#pragma unroll
+            for (int v = 0; v < 9; ++v) A.FS[(size_t)((2 * d + side) * 9 + v) * I.n + c] = f.v[v];
+        }
+    }
+}
+template <class R> GMT_HD void adj_recon_prim_cell(const AdjArgs<R>& A, const R* Q, size_t c) {
+    const Idx<R> I = idx_of(A);
+    const size_t n = I.n;
+    const Consts<R>& K = A.K;
+    const bool mm = A.recon == RECON_MINMOD;
+    int x, y, z;
+    cell_xyz(A, c, x, y, z);
+    size_t cs[7];
+    stencil7(I, x, y, z, cs);
+    const Q9<R> m0 = fs_get(Q, n, c, 0);
+    const Q9<R> uh = prim_hancock(Q, n, m0, cs, A.dtdx, K.gamma, mm);
+    R mh0, mh4;       // density and pressure of the predictor decide which interface states reverted
+    bool hrev;
+    {
+        const Q9<R> mh = cons2prim(uh, K.gamma, K.smallr, K.pfl);
+        hrev = mh.v[0] <= K.smallr || mh.v[4] <= K.pfl;
+        mh0 = hrev ? m0.v[0] : mh.v[0];
+        mh4 = hrev ? m0.v[4] : mh.v[4];
+    }
+    // the interface states: f = mh +- s_d, or m0 where reverted
+    Q9<R> m0b = q9_zero<R>(), mhb = q9_zero<R>();
+    unsigned bad = 0;
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) {
+        const size_t cl = d == 0 ? cs[1] : (d == 1 ? cs[3] : cs[5]), cr = d == 0 ? cs[2] : (d == 1 ? cs[4] : cs[6]);
+        R s0, s4;
+        {
+            const R l0 = m0.v[0] - Q[cl], r0 = Q[cr] - m0.v[0];
+            const R l4 = m0.v[4] - Q[4 * n + cl], r4 = Q[4 * n + cr] - m0.v[4];
+            s0 = mm ? R(0.5) * minmod(l0, r0) : R(0.5) * moncen(l0, r0);
+            s4 = mm ? R(0.5) * minmod(l4, r4) : R(0.5) * moncen(l4, r4);
+        }
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const R a = side ? R(-1) : R(1);
+            const bool b = A.iflo && (mh0 + a * s0 < K.smallr || mh4 + a * s4 < K.pfl);
+            const Q9<R> fb = fs_get(A.FSb, n, c, 2 * d + side);
+            bad |= (b ? 1u : 0u) << (2 * d + side);
+#pragma unroll
+            for (int v = 0; v < 9; ++v) {
+                if (b) m0b.v[v] += fb.v[v];
+                else mhb.v[v] += fb.v[v];
+            }
+        }
+    }
+    // predictor: mh = c2p(p2c(m0) - h sum_d [F_d(m0 + s_d) - F_d(m0 - s_d)]), or m0 if reverted
+    Q9<R> Fb = q9_zero<R>();   // stays zero when the predictor reverted
+    if (hrev) {
+        q9_add(m0b, mhb);
+    } else {
+        Q9<R> uhb = q9_zero<R>();
+        cons2prim_adj(uh, K.gamma, K.smallr, K.pfl, mhb, uhb);
+        prim2cons_adj(m0, K.gamma, uhb, m0b);
+        const R h = R(0.5) * A.dtdx;
+#pragma unroll
+        for (int v = 0; v < 9; ++v) Fb.v[v] = -h * uhb.v[v];
+    }
+    // per direction: the slope's adjoint, the two fluxes' vector-Jacobian products, the limiter.  m0 gets
+    // (gl - gr) sbar, the neighbours -gl sbar, +gr sbar
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) {
+        const size_t cl = d == 0 ? cs[1] : (d == 1 ? cs[3] : cs[5]), cr = d == 0 ? cs[2] : (d == 1 ? cs[4] : cs[6]);
+        Q9<R> dl, dr, sl, sb;
+        prim_slope(Q, n, m0, cl, cr, mm, dl, dr, sl);
+        {
+            const bool bp = (bad >> (2 * d)) & 1u, bm = (bad >> (2 * d + 1)) & 1u;
+            const Q9<R> fp = fs_get(A.FSb, n, c, 2 * d), fm = fs_get(A.FSb, n, c, 2 * d + 1);
+#pragma unroll
+            for (int v = 0; v < 9; ++v) sb.v[v] = (bp ? R(0) : fp.v[v]) - (bm ? R(0) : fm.v[v]);
+        }
+        const Q9<R> Fbx = rot_to_d(Fb, d);
+#pragma unroll 1
+        for (int side = 0; side < 2; ++side) {
+            const R a = side ? R(-1) : R(1);
+            Q9<R> jx = q9_zero<R>();
+            phys_flux_x_adj(rot_to_d(padd(m0, sl, a), d), K.gamma, Fbx, jx);
+            const Q9<R> j = rot_from_d(jx, d);
+#pragma unroll
+            for (int v = 0; v < 9; ++v) {
+                m0b.v[v] += a * j.v[v];
+                sb.v[v] += j.v[v];
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < 9; ++v) {
+            R gl, gr;
+            slope_deriv(dl.v[v], dr.v[v], mm, gl, gr);
+            const R Ad = sb.v[v] * gl, Bd = sb.v[v] * gr;
+            m0b.v[v] += Ad - Bd;
+            A.QB[(size_t)(9 + 9 * d + v) * n + c] = Ad;
+            A.QB[(size_t)(36 + 9 * d + v) * n + c] = Bd;
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < 9; ++v) A.QB[(size_t)v * n + c] = m0b.v[v];
 }
 
 // pass 6: gather the primitive adjoint of cell c and map it through cons2prim

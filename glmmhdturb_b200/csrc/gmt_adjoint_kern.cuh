@@ -38,9 +38,18 @@ template <int RIEM, bool DUALS, class R> __global__ void __launch_bounds__(128, 
     const size_t n = (size_t)A.nx * A.ny * A.nz;
     GMT_ADJ_LOOP adj_riemann_cell<RIEM, DUALS>(A, c);
 }
-template <class R> __global__ void __launch_bounds__(128, 3) adj_recon_kernel(const AdjArgs<R> A) {
+// FP64: passes 1 and 5 from primitive planes Q
+template <class R> __global__ void __launch_bounds__(256) adj_prim_kernel(const AdjArgs<R> A, R* Q) {
     const size_t n = (size_t)A.nx * A.ny * A.nz;
-    GMT_ADJ_LOOP adj_recon_cell(A, c);
+    GMT_ADJ_LOOP adj_prim_cell(A, Q, c);
+}
+template <class R> __global__ void __launch_bounds__(128, 4) adj_faces_prim_kernel(const AdjArgs<R> A, const R* Q) {
+    const size_t n = (size_t)A.nx * A.ny * A.nz;
+    GMT_ADJ_LOOP adj_faces_prim_cell(A, Q, c);
+}
+template <class R> __global__ void __launch_bounds__(128, 3) adj_recon_prim_kernel(const AdjArgs<R> A, const R* Q) {
+    const size_t n = (size_t)A.nx * A.ny * A.nz;
+    GMT_ADJ_LOOP adj_recon_prim_cell(A, Q, c);
 }
 template <class R> __global__ void __launch_bounds__(128) adj_gather_kernel(const AdjArgs<R> A) {
     const size_t n = (size_t)A.nx * A.ny * A.nz;
@@ -213,7 +222,9 @@ template <class R> static void launch_recon_pass(const AdjArgs<R>& A, int nb, cu
         adj_smem_attr(adj_recon_staged_kernel<R>, sm);
         adj_recon_staged_kernel<R><<<nb, ADJ_NT, sm, s>>>(A);
     } else {
-        adj_recon_kernel<R><<<nb, 128, 0, s>>>(A);
+        // the fluxes' planes are free after pass 3 and hold the primitives
+        adj_prim_kernel<R><<<nb, 256, 0, s>>>(A, A.FL);
+        adj_recon_prim_kernel<R><<<nb, 128, 0, s>>>(A, A.FL);
     }
 }
 
@@ -274,7 +285,13 @@ template <class R> cudaError_t launch_adjoint_t(const AdjArgs<R>& A, const Unspl
     cudaError_t er = cudaErrorNotSupported;
     if (rec) er = launch_record(*rec, A.recon, A.riem, s);
     if (er == cudaErrorNotSupported) {
-        adj_faces_kernel<R><<<nb, 128, 0, s>>>(A);
+        if constexpr (std::is_same<R, double>::value) {
+            // the primitives in QB, which pass 5 is the first to write
+            adj_prim_kernel<R><<<nb, 256, 0, s>>>(A, A.QB);
+            adj_faces_prim_kernel<R><<<nb, 128, 0, s>>>(A, A.QB);
+        } else {
+            adj_faces_kernel<R><<<nb, 128, 0, s>>>(A);
+        }
         if (A.riem == RIEM_HLL) adj_flux_kernel<RIEM_HLL, R><<<nb, 128, 0, s>>>(A);
         else if (A.riem == RIEM_LLF_BOUND) adj_flux_kernel<RIEM_LLF_BOUND, R><<<nb, 128, 0, s>>>(A);
         else adj_flux_kernel<RIEM_HLLD, R><<<nb, 128, 0, s>>>(A);
