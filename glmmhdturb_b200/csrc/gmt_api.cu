@@ -587,7 +587,6 @@ int gmt_destroy(gmt_ctx* c) {
     cudaFree(c->spec);
     cudaFree(c->adj);
     cudaFree(c->adj_damp);
-    cudaFree(c->adj_err);
     if (c->cap) cudaStreamDestroy(c->cap);
     cudaFree(c->loop);
     cudaFree(c->loopc);
@@ -786,10 +785,9 @@ int gmt_adjoint_step(gmt_ctx* c, const void* u, const void* ubar_next, void* uba
     cudaStream_t s = (cudaStream_t)stream;
     if (!c->adj) {
         GMT_CUDA(cudaMalloc(&c->adj, adjoint_scratch_reals(c->n) * c->esize));
-        GMT_CUDA(cudaMalloc(&c->adj_damp, sizeof(double)));
-        GMT_CUDA(cudaMalloc(&c->adj_err, sizeof(int)));
-        GMT_CUDA(cudaMemsetAsync(c->adj_damp, 0, sizeof(double), s));
-        GMT_CUDA(cudaMemsetAsync(c->adj_err, 0, sizeof(int), s));
+        GMT_CUDA(cudaMalloc(&c->adj_damp, 2 * sizeof(double)));   // the error flag behind it: one read-back
+        c->adj_err = reinterpret_cast<int*>(c->adj_damp + 1);
+        GMT_CUDA(cudaMemsetAsync(c->adj_damp, 0, 2 * sizeof(double), s));
     }
     const double dx = p.boxlen / p.nx;
     auto go = [&](auto zero) -> int {
@@ -851,11 +849,13 @@ int gmt_adjoint_amp_grad(gmt_ctx* c, double* out, int32_t reset, void* stream) {
     if (!c || !out) return fail(GMT_ERR_ARG, "gmt_adjoint_amp_grad: null argument");
     cudaStream_t s = (cudaStream_t)stream;
     if (!c->adj_damp) { *out = 0.0; return GMT_OK; }
-    int herr = 0;
-    GMT_CUDA(cudaMemcpyAsync(out, c->adj_damp, sizeof(double), cudaMemcpyDeviceToHost, s));
-    GMT_CUDA(cudaMemcpyAsync(&herr, c->adj_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    double h[2];
+    GMT_CUDA(cudaMemcpyAsync(h, c->adj_damp, sizeof(h), cudaMemcpyDeviceToHost, s));
     if (reset) GMT_CUDA(cudaMemsetAsync(c->adj_damp, 0, sizeof(double), s));
     GMT_CUDA(cudaStreamSynchronize(s));
+    *out = h[0];
+    int herr;
+    std::memcpy(&herr, &h[1], sizeof(int));
     if (herr) {
         GMT_CUDA(cudaMemsetAsync(c->adj_err, 0, sizeof(int), s));
         GMT_CUDA(cudaStreamSynchronize(s));
@@ -1031,14 +1031,11 @@ LoopConst loop_const_of(const gmt_params& p, double alpha, double beta, double s
 template <class R>
 cudaError_t run_enqueue(gmt_ctx* c, const void* src, void* dst, int flags, cudaStream_t s) {
     const gmt_params& p = c->p;
-    tick_kernel<<<1, 32, 0, s>>>(c->loop, c->loopc, c->cfl, 1);
+    tick_kernel<<<1, 64, 0, s>>>(c->loop, c->loopc, c->cfl, c->modes, c->mode_k_dev);
     if (flags & GMT_RUN_FORCING) {
-        ou_cond_kernel<<<1, 64, 0, s>>>(c->modes, c->loop, c->loopc, c->mode_k_dev);
-        btab_cond_kernel<R><<<dim3((p.ny * p.nz + 255) / 256, 1), 256, 0, s>>>((const BoxTables<R>*)c->bt, c->loop,
+        btab_cond_kernel<R><<<dim3(std::min((p.ny * p.nz + BTAB_ROWS - 1) / BTAB_ROWS, 148 * 4), 1), 4 * BTAB_ROWS, 0, s>>>((const BoxTables<R>*)c->bt, c->loop,
                                                                               c->mode_k_dev);
     }
-    cudaError_t e = cudaMemsetAsync(c->cfl, 0, 2 * sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
     UnsplitArgs<R> A;
     A.u = cplanes<R>(src, c->n);
     A.o = planes<R>(dst, c->n);
@@ -1208,14 +1205,12 @@ template <class R> int ens_bind(gmt_ensemble* E, void* const* u, void* const* w,
 }
 
 template <class R> cudaError_t ens_enqueue(gmt_ensemble* E, int par, int flags, cudaStream_t s) {
-    tick_kernel<<<(E->nbox + 63) / 64, 64, 0, s>>>(E->loop, E->loopc, E->cfl, E->nbox);
+    tick_kernel<<<E->nbox, 64, 0, s>>>(E->loop, E->loopc, E->cfl, E->modes, E->mode_k_dev);
     if (flags & GMT_RUN_FORCING) {
-        ou_cond_kernel<<<E->nbox, 64, 0, s>>>(E->modes, E->loop, E->loopc, E->mode_k_dev);
-        btab_cond_kernel<R><<<dim3((E->rows_max + 255) / 256, E->nbox), 256, 0, s>>>((const BoxTables<R>*)E->bt, E->loop,
+        btab_cond_kernel<R><<<dim3(std::min((E->rows_max + BTAB_ROWS - 1) / BTAB_ROWS, 32), E->nbox), 4 * BTAB_ROWS, 0, s>>>((const BoxTables<R>*)E->bt, E->loop,
                                                                                      E->mode_k_dev);
     }
-    cudaError_t e = cudaMemsetAsync(E->cfl, 0, 2 * E->nbox * sizeof(unsigned long long), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(E->queue + par, 0, sizeof(unsigned), s);
+    cudaError_t e = cudaMemsetAsync(E->queue + par, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     const UnsplitArgs<R>* args = static_cast<const UnsplitArgs<R>*>(E->args) + par * E->nbox;
     int riem = E->p.riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : E->p.riemann;

@@ -388,15 +388,13 @@ cudaError_t launch_ou_update(double* modes, uint32_t seed, uint32_t counter, dou
 template <class R>
 __global__ void __launch_bounds__(256) btab_kernel(const double* modes, const R* trigy, const R* trigz, int ny, int nz,
                                                    R* btab) {
-    int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= ny * nz) return;
-    btab_row(modes, c_mode_k, trigy, trigz, ny, nz, row % ny, row / ny, btab + (size_t)row * 24);
+    btab_rows(modes, c_mode_k, trigy, trigz, ny, nz, (int)blockIdx.x * BTAB_ROWS, btab);
 }
 
 template <class R>
 cudaError_t launch_btab(const double* modes, const R* trigy, const R* trigz, int ny, int nz, R* btab, cudaStream_t s) {
     int rows = ny * nz;
-    btab_kernel<R><<<(rows + 255) / 256, 256, 0, s>>>(modes, trigy, trigz, ny, nz, btab);
+    btab_kernel<R><<<(rows + BTAB_ROWS - 1) / BTAB_ROWS, 4 * BTAB_ROWS, 0, s>>>(modes, trigy, trigz, ny, nz, btab);
     return cudaGetLastError();
 }
 
