@@ -241,15 +241,15 @@ template <class R, int RECON, int RIEM> struct AdjRecordScheme : UnsplitScheme<R
         finish_update_adj(r1, K, glm_fac, turb, ax, ay, az, dt, ob, rb, ab);
     }
 };
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX, int TOY>
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX, int TOY, bool OVER>
 __global__ void __launch_bounds__(MAXT, MINB) adj_record_kernel(const __grid_constant__ UnsplitArgs<R> A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    scheme_tile<R, AdjRecordScheme<R, RECON, RIEM>, TOX, TOY, false, true>(A, step_vals(A), blockIdx.x, blockIdx.y,
-                                                                            blockIdx.z, smem_raw);
+    scheme_tile<R, AdjRecordScheme<R, RECON, RIEM>, TOX, TOY, OVER>(A, step_vals(A), blockIdx.x, blockIdx.y,
+                                                                                  blockIdx.z, smem_raw);
 }
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX, int TOY>
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX, int TOY, bool OVER>
 static cudaError_t record_go(const UnsplitArgs<R>& A, cudaStream_t s) {
-    auto k = adj_record_kernel<R, RECON, RIEM, MAXT, MINB, TOX, TOY>;
+    auto k = adj_record_kernel<R, RECON, RIEM, MAXT, MINB, TOX, TOY, OVER>;
     static int configured[64] = {0};
     {
         cudaError_t e = configure_once(k, configured);
@@ -257,13 +257,15 @@ static cudaError_t record_go(const UnsplitArgs<R>& A, cudaStream_t s) {
     }
     const int nt = A.ox * A.oy;
     if (nt > MAXT || nt < 1) return cudaErrorInvalidConfiguration;
-    dim3 grid(A.nx / A.ox, A.ny / A.oy, (A.nz + A.lz - 1) / A.lz);
+    dim3 grid((A.nx + A.ox - 1) / A.ox, (A.ny + A.oy - 1) / A.oy, (A.nz + A.lz - 1) / A.lz);
     k<<<grid, nt, unsplit_smem_bytes<R>(A.ox, A.oy), s>>>(A);
     return cudaGetLastError();
 }
 template <class R, int RECON, int RIEM> static cudaError_t record_tile(const UnsplitArgs<R>& A, cudaStream_t s) {
-    if (A.ox == 32 && A.oy == 16) return record_go<R, RECON, RIEM, 512, 1, 32, 16>(A, s);
-    return record_go<R, RECON, RIEM, 512, 1, 0, 0>(A, s);
+    if (A.ox == 32 && A.oy == 16)
+        return overhangs(A) ? record_go<R, RECON, RIEM, 512, 1, 32, 16, true>(A, s)
+                            : record_go<R, RECON, RIEM, 512, 1, 32, 16, false>(A, s);
+    return record_go<R, RECON, RIEM, 512, 1, 0, 0, true>(A, s);
 }
 // passes 1-3 by the record tile, FP32, for PLM-MC / minmod with HLLD (also its LLF forms) or HLL;
 // cudaErrorNotSupported otherwise (the caller then runs the per-cell passes).  In FP64 the three

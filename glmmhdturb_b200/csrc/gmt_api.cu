@@ -69,6 +69,17 @@ double forcing_sigma0(double amp, double alpha, double beta) {
     return amp * std::sqrt((1.0 - alpha * alpha) / (8.0 * beta * beta * s));
 }
 
+// Streams that the boxes of an ensemble fork over, one box each where there are enough.  A box's kernel
+// fills the chip for a part of its time only; with all boxes queued, blocks of others take the SMs it
+// leaves idle (64 uneven boxes, 41 M zones: 4.22 ms a step over 8 streams, 3.83 over 32, 3.65 over 64).
+// The single-box kernels run here, with a box's arguments in constant memory: a persistent kernel over
+// a queue of tiles of all boxes held them in registers, spilled, and took 3.95 ms.
+constexpr int ENS_LANES = 64;
+// Mean box below which two steps are replayed as a graph: a box's three launches take the host 7 us, about
+// what a 48^3 box takes the chip (64 boxes); above that plain launches keep the boxes' order, which the
+// graph's branches do not (41 M zones: 3.65 ms a step against 3.75 to 3.93).
+constexpr size_t ENS_GRAPH_ZONES = (size_t)48 * 48 * 48;
+
 bool divides(int n, int t) { return t > 0 && n % t == 0; }
 
 }  // namespace
@@ -109,8 +120,8 @@ struct gmt_ctx {
     int adj_percell = 0;           // 1: the adjoint runs its first three passes per cell
     long long wait_cycles = GMT_WAIT_CYCLES;   // budget of the tile kernels' bounded waits
     int wait_test = 0;             // failure-path tests: staging withheld, so every bounded wait runs out
-    struct TmaMap { const void* base; CUtensorMap map; };
-    TmaMap tma[2] = {};            // tensor maps of the last two input states (tile staging)
+    struct TmaMap { const void* base; int ox, oy; CUtensorMap map; };
+    TmaMap tma[4] = {};            // tensor maps of the last input states and tiles (tile staging)
     int tma_next = 0;
     struct CtTmaMap { const void* base; CUtensorMap map8, map1; };
     CtTmaMap ct_tma[2] = {};       // the same for the CT state (8 variables, and bzf alone)
@@ -132,43 +143,52 @@ template <class R> Consts<R> consts_of(const gmt_params& p) {
     return K;
 }
 
+// The z chunk that fills the chip best: the number of rounds of blocks over the 148 SMs times the
+// length of a block.  Short chunks repeat the fixed part, long ones leave SMs idle in the last round;
+// with more than one round a share of a block's time is added, because blocks do not end together.
+// (FP32 MC + HLLD, chunk -> us: 64^3 4 -> 41, 8 -> 66; 96^3 12 -> 92, 6 -> 105; 192^3 32 -> 694,
+// 6 -> 833; 256^3 32 -> 1549, 16 -> 1623; 512^3 128 -> 11.59 ms, 64 and 256 -> 11.70 ms; the second
+// figures of the first four are the chunks of a rule that only asked for eight rounds of blocks.)
+int choose_chunk(long cols, int nz) {
+    // a block takes lz planes and 2.8 planes' time for its start and for the first and last planes, which
+    // only reconstruct (64^3, chunk 4 -> 64: 41 -> 401 us, 6.05 us a plane)
+    constexpr double start = 2.8;
+    double best = 1e300;
+    int last = 0, choice = nz;
+    for (int nch = 1; nch <= std::min(nz, 4096); ++nch) {
+        const int lz = (nz + nch - 1) / nch;
+        if (lz == last) continue;
+        last = lz;
+        const long rounds = (cols * ((nz + lz - 1) / lz) + 147) / 148;
+        const double cost = ((double)rounds + (rounds > 1 ? 0.2 : 0.0)) * (lz + start);
+        if (cost < best) { best = cost; choice = lz; }
+    }
+    return choice;
+}
+
 int choose_tile(gmt_ctx* c, bool ct = false) {
     const gmt_params& p = c->p;
     const int maxt = ct ? ct_max_threads(c->esize) : unsplit_max_threads(c->esize);
     auto smem = [&](int ox, int oy) { return ct ? ct_smem_of(c->esize, ox, oy) : unsplit_smem(c->esize, ox, oy); };
-    // largest first: 32x16 (512 threads, one block per SM) measured fastest at 512^3 FP32 for
-    // both the unsplit and the march scheme; FP64 stops at 256 threads
-    static const int cand[][2] = {{32, 16}, {32, 8}, {32, 4}, {16, 8}, {16, 4}, {8, 8}, {8, 4}, {4, 4},
-                                  {8, 2}, {4, 2}, {2, 2}, {8, 1}, {4, 1}, {2, 1}, {1, 1}};
+    auto cols = [&](int ox, int oy) { return (long)((p.nx + ox - 1) / ox) * ((p.ny + oy - 1) / oy); };
     int ox = p.tile_x, oy = p.tile_y;
-    auto fits = [&](int tx, int ty) {
-        return divides(p.nx, tx) && divides(p.ny, ty) && tx * ty <= maxt && smem(tx, ty) <= 227 * 1024;
-    };
     if (ox <= 0 || oy <= 0) {
-        ox = oy = 0;
-        if (!ct && c->esize == 8 && fits(16, 16)) {
-            // the FP64 step: 16x16 (a compile-time tile) has less halo than 32x8 and measured
-            // 3.8 % faster at 512^3 than the runtime 32x8 tile
-            ox = oy = 16;
+        // the last tiles of a row and column may overhang the box, so the tile need not divide it
+        if (c->esize == 8) {
+            // FP64: 16x16, which has less halo than 32x8 (512^3: 3.8 % faster); CT's rings leave room for 16x8
+            ox = 16;
+            oy = ct ? 8 : 16;
         } else {
-            for (auto& t : cand)
-                if (fits(t[0], t[1])) {
-                    ox = t[0];
-                    oy = t[1];
-                    break;
-                }
+            ox = 32;
+            oy = 16;
         }
+    } else {
+        if (!divides(p.nx, ox) || !divides(p.ny, oy))
+            return fail(GMT_ERR_ARG, "tile " + std::to_string(ox) + "x" + std::to_string(oy) + " does not divide the grid");
+        if (ox * oy > maxt) return fail(GMT_ERR_ARG, "tile_x*tile_y must be <= " + std::to_string(maxt));
+        if (smem(ox, oy) > 227 * 1024) return fail(GMT_ERR_ARG, "tile needs more than 227 KB shared memory");
     }
-    if (!divides(p.nx, ox) || !divides(p.ny, oy))
-        return fail(GMT_ERR_ARG, "tile " + std::to_string(ox) + "x" + std::to_string(oy) + " does not divide the grid");
-    if (ox * oy > maxt) return fail(GMT_ERR_ARG, "tile_x*tile_y must be <= " + std::to_string(maxt));
-    if (smem(ox, oy) > 227 * 1024) return fail(GMT_ERR_ARG, "tile needs more than 227 KB shared memory");
-    int lz = p.tile_z;
-    if (lz <= 0) {
-        long cols = (long)(p.nx / ox) * (p.ny / oy);
-        lz = p.nz;
-        while (lz > 8 && cols * ((p.nz + lz - 1) / lz) < 148L * 8) lz = (lz + 1) / 2;
-    }
+    const int lz = p.tile_z > 0 ? p.tile_z : choose_chunk(cols(ox, oy), p.nz);
     c->ox = ox; c->oy = oy; c->lz = std::min(lz, p.nz);
     return GMT_OK;
 }
@@ -227,28 +247,42 @@ const R* tma_base(const P& planes, int nvar, int nx, int ny, int nz, int ox, int
     return base;
 }
 
-template <class R> void set_tma(gmt_ctx* c, UnsplitArgs<R>& A) {
+// the planes can be staged in 16-byte quads: rows and tiles of whole quads, every plane 16-byte aligned
+template <class R> int quad_ok(const R* const* planes, int nvar, int nx, int ox) {
+    constexpr int Q = 16 / (int)sizeof(R);
+    if (nx % Q != 0 || ox % Q != 0) return 0;
+    for (int v = 0; v < nvar; ++v)
+        if (reinterpret_cast<uintptr_t>(planes[v]) % 16 != 0) return 0;
+    return 1;
+}
+
+// A's staging: quads, and the tensor map of its input state (false: no map can be made)
+template <class R> bool set_staging(UnsplitArgs<R>& A) {
+    A.quad = quad_ok<R>(A.u.p, 9, A.nx, A.ox);
     A.use_tma = 0;
     std::memset(&A.tmap, 0, sizeof(A.tmap));
     const R* base = tma_base<R>(A.u, 9, A.nx, A.ny, A.nz, A.ox, A.oy, 4);
-    if (!base) return;
+    if (base && encode_state_map(&A.tmap, base, A.nx, A.ny, A.nz, 9, A.ox + 8, A.oy + 4, 9)) A.use_tma = 1;
+    return A.use_tma != 0;
+}
+// the same with the context's maps of its last input states
+template <class R> void set_tma(gmt_ctx* c, UnsplitArgs<R>& A) {
+    const R* base = tma_base<R>(A.u, 9, A.nx, A.ny, A.nz, A.ox, A.oy, 4);
     for (const gmt_ctx::TmaMap& t : c->tma)
-        if (t.base == base) {
+        if (base && t.base == base && t.ox == A.ox && t.oy == A.oy) {
+            A.quad = quad_ok<R>(A.u.p, 9, A.nx, A.ox);
             A.tmap = t.map;
             A.use_tma = 1;
             return;
         }
-    CUtensorMap m;
-    if (!encode_state_map(&m, base, A.nx, A.ny, A.nz, 9, A.ox + 8, A.oy + 4, 9)) return;
-    c->tma[c->tma_next].base = base;
-    c->tma[c->tma_next].map = m;
-    c->tma_next ^= 1;
-    A.tmap = m;
-    A.use_tma = 1;
+    if (!set_staging(A)) return;
+    c->tma[c->tma_next] = {base, A.ox, A.oy, A.tmap};
+    c->tma_next = (c->tma_next + 1) & 3;
 }
 
 // CT: the staged region is (ox+8) x (oy+5) cells; one map moves the 8 state variables, one bzf
 template <class R> void set_ct_tma(gmt_ctx* c, CTArgs<R>& A) {
+    A.quad = quad_ok<R>(A.q.p, 8, A.nx, A.ox);
     A.use_tma = 0;
     std::memset(&A.tmap8, 0, sizeof(A.tmap8));
     std::memset(&A.tmap1, 0, sizeof(A.tmap1));
@@ -838,7 +872,7 @@ int gmt_adjoint_step(gmt_ctx* c, const void* u, const void* ubar_next, void* uba
         T.rec_ub = A.ub.p[0];
         T.rec_damp = A.damp;
         T.rec_amp = A.amp;
-        const bool record = c->ox > 0 && c->oy > 0 && c->lz > 0 && !c->adj_percell;
+        const bool record = !c->adj_percell;
         cudaError_t e = launch_adjoint<R>(A, record ? &T : nullptr, s);
         return e == cudaSuccess ? GMT_OK : cuda_fail(e, "gmt_adjoint_step");
     };
@@ -1134,20 +1168,12 @@ int gmt_run(gmt_ctx* c, void* u, void* w, int32_t nsteps, double t0, double t_en
 // ------------------------------------------------------------------------------------------
 }  // extern "C"
 
-// z-chunk of a box's ensemble work items: the box's nz split into ceil(n/64) equal chunks, so the
-// per-chunk prologue (two extra planes) stays near 3-6% while a 64-box ensemble still yields
-// thousands of items for the persistent grid
-inline int ens_lz(int n) {
-    const int nch = (n + 63) / 64;
-    return (n + nch - 1) / nch;
-}
-
 struct gmt_ensemble {
     gmt_params p;
     int nbox = 0;
     int esize = 4;
-    int nsm = 148;
-    std::vector<int> n;
+    std::vector<int> n, ox, lz;      // per box: grid size, tile width, z chunk
+    std::vector<int> order;          // boxes, the longest blocks first: box order[j] runs on lane j % lanes
     std::vector<double> amp;
     std::vector<uint32_t> seed;
     LoopState* loop = nullptr;       // [nbox]
@@ -1155,25 +1181,71 @@ struct gmt_ensemble {
     unsigned long long* cfl = nullptr;  // [2 nbox]
     double* modes = nullptr;         // [nbox][61][3][2]
     std::vector<void*> btab, trig;   // per box: row table; trig x, y, z
+    std::vector<void*> trig8;        // per box, FP32: the x table of force_accel_f32
     void* bt = nullptr;              // BoxTables<R>[nbox]
-    void* args = nullptr;            // UnsplitArgs<R>[2][nbox]
-    EnsItem* items = nullptr;
-    int nitems = 0;
-    unsigned* queue = nullptr;       // [2] one counter per parity
+    std::vector<UnsplitArgs<float>> a32;   // kernel arguments, [2 parities][nbox]
+    std::vector<UnsplitArgs<double>> a64;
+    // the boxes' kernels of a step are independent: they fork from the caller's stream over these
+    std::vector<cudaStream_t> lane;
+    std::vector<cudaEvent_t> lane_ev;
+    cudaEvent_t fork = nullptr;
     int* err = nullptr;
     const int* mode_k_dev = nullptr;
     cudaStream_t cap = nullptr;
     std::vector<const void*> bound_u, bound_w;
     cudaGraphExec_t exec = nullptr;
     int exec_flags = -1;
-    int rows_max = 0;
     std::vector<double> alpha, beta, sigma0;
 };
 
 namespace {
 
-template <class R> int ens_bind(gmt_ensemble* E, void* const* u, void* const* w, int flags) {
-    std::vector<UnsplitArgs<R>> A(2 * E->nbox);
+std::vector<UnsplitArgs<float>>& ens_args(gmt_ensemble* E, float) { return E->a32; }
+std::vector<UnsplitArgs<double>>& ens_args(gmt_ensemble* E, double) { return E->a64; }
+
+// Tiles and chunks of the boxes.  FP32: 32x16 tiles, or 16x16 (two blocks share an SM, the pair 14 %
+// slower than a 32x16 block) where the box width leaves the wide tile's last column mostly empty.  All
+// boxes share the longest chunk allowed, the one that costs least when the blocks of the whole
+// ensemble are spread over the chip: short chunks repeat the 2.8 planes of a block's start, long ones
+// leave a longer tail.
+void ens_tiles(gmt_ensemble* E) {
+    const int nb = E->nbox;
+    E->ox.resize(nb);
+    E->lz.resize(nb);
+    std::vector<double> load(nb);   // blocks of one chunk, in 32x16 blocks
+    E->order.resize(nb);
+    for (int b = 0; b < nb; ++b) E->order[b] = b;
+    for (int b = 0; b < nb; ++b) {
+        const int n = E->n[b];
+        const double wide = (double)((n + 31) / 32) * (n / 16), half = (double)(n / 16) * (n / 16) * 0.57;
+        E->ox[b] = E->esize == 8 || half < wide ? 16 : 32;
+        load[b] = std::min(wide, half);
+    }
+    double best = 1e300;
+    for (int top = 4; top <= 256; top *= 2) {
+        double work = 0.0, tail = 0.0;
+        for (int b = 0; b < nb; ++b) {
+            const int nch = (E->n[b] + top - 1) / top, lz = (E->n[b] + nch - 1) / nch;
+            work += load[b] * nch * (lz + 2.8);
+            tail = std::max(tail, lz + 2.8);
+        }
+        const double cost = std::max(work / 148.0, tail) + 0.5 * tail;
+        if (cost >= best) continue;
+        best = cost;
+        for (int b = 0; b < nb; ++b) {
+            const int nch = (E->n[b] + top - 1) / top;
+            E->lz[b] = (E->n[b] + nch - 1) / nch;
+        }
+    }
+    // longest blocks first
+    std::stable_sort(E->order.begin(), E->order.end(), [&](int a, int b) {
+        return E->lz[a] != E->lz[b] ? E->lz[a] > E->lz[b] : E->n[a] > E->n[b];
+    });
+}
+
+template <class R> void ens_bind(gmt_ensemble* E, void* const* u, void* const* w, int flags) {
+    std::vector<UnsplitArgs<R>>& A = ens_args(E, R(0));
+    A.assign(2 * E->nbox, UnsplitArgs<R>{});
     for (int par = 0; par < 2; ++par)
         for (int b = 0; b < E->nbox; ++b) {
             UnsplitArgs<R>& a = A[par * E->nbox + b];
@@ -1182,43 +1254,63 @@ template <class R> int ens_bind(gmt_ensemble* E, void* const* u, void* const* w,
             a.u = cplanes<R>(par == 0 ? u[b] : w[b], cells);
             a.o = planes<R>(par == 0 ? w[b] : u[b], cells);
             a.nx = a.ny = a.nz = n;
-            a.ox = ens_tile_x<R>(); a.oy = 16; a.lz = ens_lz(n);
-            a.dt = a.dtdx = a.ch = a.glm_fac = a.ramp = R(0);
+            a.ox = E->ox[b]; a.oy = 16; a.lz = E->lz[b];
             a.K = consts_of<R>(E->p);
             a.iflo = E->p.iflo; a.use_llf = E->p.riemann == GMT_RIEMANN_LLF;
             a.do_turb = (flags & GMT_RUN_FORCING) ? 1 : 0;
             a.btab = a.do_turb ? static_cast<const R*>(E->btab[b]) : nullptr;
             a.trigx = static_cast<const R*>(E->trig[3 * b]);
-            a.trig8 = nullptr;   // the ensemble kernel reads the generic tables (force_accel)
+            a.trig8 = static_cast<const R*>(E->trig8[b]);
             a.cfl_out = E->cfl + 2 * b;
             a.err = E->err;
             a.wait_cycles = GMT_WAIT_CYCLES;
-            a.wait_test = 0;
             a.dx = (R)(E->p.boxlen / n);
             a.dparams = reinterpret_cast<const double*>(E->loop + b);
-            a.fmass = nullptr;
-            a.use_tma = 0;   // the ensemble kernel stages by cp.async
-            std::memset(&a.tmap, 0, sizeof(a.tmap));
+            set_staging(a);
         }
-    cudaError_t e = cudaMemcpy(E->args, A.data(), A.size() * sizeof(UnsplitArgs<R>), cudaMemcpyHostToDevice);
-    return e == cudaSuccess ? GMT_OK : cuda_fail(e, "ensemble bind");
 }
 
-template <class R> cudaError_t ens_enqueue(gmt_ensemble* E, int par, int flags, cudaStream_t s) {
-    tick_kernel<<<E->nbox, 64, 0, s>>>(E->loop, E->loopc, E->cfl, E->modes, E->mode_k_dev);
-    if (flags & GMT_RUN_FORCING) {
-        btab_cond_kernel<R><<<dim3(std::min((E->rows_max + BTAB_ROWS - 1) / BTAB_ROWS, 32), E->nbox), 4 * BTAB_ROWS, 0, s>>>((const BoxTables<R>*)E->bt, E->loop,
-                                                                                     E->mode_k_dev);
+// f() puts the boxes' work on the lanes, which are forked from s and joined to it again
+template <class F> cudaError_t ens_fork(gmt_ensemble* E, cudaStream_t s, F f) {
+    const int L = (int)E->lane.size();
+    cudaError_t e = cudaEventRecord(E->fork, s);
+    for (int i = 0; e == cudaSuccess && i < L; ++i) e = cudaStreamWaitEvent(E->lane[i], E->fork, 0);
+    if (e == cudaSuccess) e = f();
+    for (int i = 0; i < L; ++i) {   // joined in any case: a lane left out would break a capture
+        const cudaError_t e1 = cudaEventRecord(E->lane_ev[i], E->lane[i]);
+        const cudaError_t e2 = cudaStreamWaitEvent(s, E->lane_ev[i], 0);
+        if (e == cudaSuccess) e = e1 != cudaSuccess ? e1 : e2;
     }
-    cudaError_t e = cudaMemsetAsync(E->queue + par, 0, sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
-    const UnsplitArgs<R>* args = static_cast<const UnsplitArgs<R>*>(E->args) + par * E->nbox;
-    int riem = E->p.riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : E->p.riemann;
-    return launch_ensemble(args, E->items, E->nitems, E->queue + par, E->p.recon, riem, E->nsm, s);
+    return e;
 }
 
-cudaError_t ens_enqueue_any(gmt_ensemble* E, int par, int flags, cudaStream_t s) {
-    return E->esize == 8 ? ens_enqueue<double>(E, par, flags, s) : ens_enqueue<float>(E, par, flags, s);
+// One step of every box, each on its lane and ordered only after that box's own previous step: the boxes
+// are independent, so no box waits for the slowest one and the chip is short of blocks only at the end
+// of a run, not of every step.
+// With `first`, a box's own CFL reduction of its state u[b] goes ahead of its step.
+template <class R> cudaError_t ens_enqueue(gmt_ensemble* E, int par, int flags, bool first) {
+    const int riem = E->p.riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : E->p.riemann, L = (int)E->lane.size();
+    const std::vector<UnsplitArgs<R>>& A = ens_args(E, R(0));
+    cudaError_t e = cudaSuccess;
+    for (int j = 0; e == cudaSuccess && j < E->nbox; ++j) {
+        const int b = E->order[j];
+        const cudaStream_t s = E->lane[j % L];
+        if (first) {
+            const UnsplitArgs<R>& a = A[par * E->nbox + b];
+            e = launch_cfl<R>(a.u, (size_t)a.nx * a.ny * a.nz, a.K, E->cfl + 2 * b, s);
+            if (e != cudaSuccess) break;
+        }
+        tick_kernel<<<1, 64, 0, s>>>(E->loop + b, E->loopc + b, E->cfl + 2 * b, E->modes + (size_t)b * NMODES * 6, E->mode_k_dev);
+        if (flags & GMT_RUN_FORCING)
+            btab_cond_kernel<R><<<std::min((E->n[b] * E->n[b] + BTAB_ROWS - 1) / BTAB_ROWS, 32), 4 * BTAB_ROWS, 0, s>>>(
+                (const BoxTables<R>*)E->bt + b, E->loop + b, E->mode_k_dev);
+        e = launch_unsplit(A[par * E->nbox + b], E->p.recon, riem, s);
+    }
+    return e;
+}
+
+cudaError_t ens_enqueue_any(gmt_ensemble* E, int par, int flags, bool first) {
+    return E->esize == 8 ? ens_enqueue<double>(E, par, flags, first) : ens_enqueue<float>(E, par, flags, first);
 }
 
 }  // namespace
@@ -1229,6 +1321,12 @@ int gmt_ensemble_destroy(gmt_ensemble* E) {
     if (!E) return GMT_OK;
     if (E->exec) cudaGraphExecDestroy(E->exec);
     if (E->cap) cudaStreamDestroy(E->cap);
+    for (cudaStream_t l : E->lane)
+        if (l) cudaStreamDestroy(l);
+    for (cudaEvent_t v : E->lane_ev)
+        if (v) cudaEventDestroy(v);
+    if (E->fork) cudaEventDestroy(E->fork);
+    for (void* x : E->trig8) cudaFree(x);
     cudaFree(E->loop);
     cudaFree(E->loopc);
     cudaFree(E->cfl);
@@ -1236,9 +1334,6 @@ int gmt_ensemble_destroy(gmt_ensemble* E) {
     for (void* x : E->btab) cudaFree(x);
     for (void* x : E->trig) cudaFree(x);
     cudaFree(E->bt);
-    cudaFree(E->args);
-    cudaFree(E->items);
-    cudaFree(E->queue);
     cudaFree(E->err);
     delete E;
     return GMT_OK;
@@ -1271,9 +1366,7 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
     E->n.assign(n, n + nbox);
     E->amp.resize(nbox);
     E->seed.resize(nbox);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&E->nsm, cudaDevAttrMultiProcessorCount, dev);
+    (void)encode_tiled_fn();
     cudaError_t e = cudaSuccess;
     auto A = [&](void** ptr, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(ptr, bytes);
@@ -1283,34 +1376,25 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
     A((void**)&E->cfl, 2 * nbox * sizeof(unsigned long long));
     A((void**)&E->modes, (size_t)nbox * NMODES * 6 * sizeof(double));
     A(&E->bt, nbox * sizeof(BoxTables<double>));
-    A(&E->args, 2 * nbox * sizeof(UnsplitArgs<double>));
-    A((void**)&E->queue, 2 * sizeof(unsigned));
     A((void**)&E->err, sizeof(int));
     E->btab.assign(nbox, nullptr);
     E->trig.assign(3 * nbox, nullptr);
+    E->trig8.assign(nbox, nullptr);
     for (int b = 0; b < nbox; ++b) {
         A(&E->btab[b], (size_t)n[b] * n[b] * 24 * E->esize);
         for (int a = 0; a < 3; ++a) A(&E->trig[3 * b + a], (size_t)8 * n[b] * E->esize);
-        E->rows_max = std::max(E->rows_max, n[b] * n[b]);
+        if (E->esize == 4) A(&E->trig8[b], (size_t)8 * n[b] * 4);
     }
 
-    // work items: biggest boxes first, tiles of ens_tile_x x 16 columns (a box whose width is not a
-    // multiple of the tile gets an overhanging last tile) x ens_lz-plane chunks (the last chunk of
-    // a box may be shorter)
-    const int etx = E->esize == 8 ? ens_tile_x<double>() : ens_tile_x<float>();
-    std::vector<int> order(nbox);
-    for (int b = 0; b < nbox; ++b) order[b] = b;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return n[a] > n[b]; });
-    std::vector<EnsItem> items;
-    for (int b : order) {
-        const int lz = ens_lz(n[b]);
-        for (int bz = 0; bz < (n[b] + lz - 1) / lz; ++bz)
-            for (int by = 0; by < n[b] / 16; ++by)
-                for (int bx = 0; bx < (n[b] + etx - 1) / etx; ++bx) items.push_back({b, bx, by, bz});
+    ens_tiles(E);
+    const int lanes = std::min(nbox, ENS_LANES);
+    E->lane.assign(lanes, nullptr);
+    E->lane_ev.assign(lanes, nullptr);
+    for (int i = 0; i < lanes; ++i) {
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&E->lane[i], cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&E->lane_ev[i], cudaEventDisableTiming);
     }
-    E->nitems = (int)items.size();
-    A((void**)&E->items, items.size() * sizeof(EnsItem));
-    if (e == cudaSuccess) e = cudaMemcpy(E->items, items.data(), items.size() * sizeof(EnsItem), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&E->fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMemset(E->err, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(E->modes, 0, (size_t)nbox * NMODES * 6 * sizeof(double));
     if (e == cudaSuccess) e = mode_table_device(&E->mode_k_dev);
@@ -1332,7 +1416,10 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
                 e = cudaMemcpy(E->trig[3 * b + a], f.data(), f.size() * 4, cudaMemcpyHostToDevice);
             }
         }
-
+        if (e == cudaSuccess && E->esize == 4) {
+            std::vector<float> t8 = trig8_table(t, n[b]);
+            e = cudaMemcpy(E->trig8[b], t8.data(), t8.size() * 4, cudaMemcpyHostToDevice);
+        }
         E->amp[b] = amp ? amp[b] : base->turb_amp;
         E->seed[b] = seeds ? seeds[b] : base->turb_seed + (uint32_t)b;
         gmt_params pb = *base;
@@ -1375,8 +1462,8 @@ int gmt_ensemble_run(gmt_ensemble* E, void* const* u, void* const* w, int32_t ns
     for (int b = 0; !rebind && b < nb; ++b) rebind = E->bound_u[b] != u[b] || E->bound_w[b] != w[b];
     if (rebind) {
         GMT_CUDA(cudaStreamSynchronize(s));
-        int rc = E->esize == 8 ? ens_bind<double>(E, u, w, flags) : ens_bind<float>(E, u, w, flags);
-        if (rc) return rc;
+        if (E->esize == 8) ens_bind<double>(E, u, w, flags);
+        else ens_bind<float>(E, u, w, flags);
         E->bound_u.assign(u, u + nb);
         E->bound_w.assign(w, w + nb);
         if (E->exec) { cudaGraphExecDestroy(E->exec); E->exec = nullptr; }
@@ -1396,37 +1483,36 @@ int gmt_ensemble_run(gmt_ensemble* E, void* const* u, void* const* w, int32_t ns
     GMT_CUDA(cudaStreamSynchronize(s));
     for (auto& x : S) x.t_end = t_end;
     GMT_CUDA(cudaMemcpyAsync(E->loop, S.data(), nb * sizeof(LoopState), cudaMemcpyHostToDevice, s));
-    for (int b = 0; b < nb; ++b) {
-        const size_t cells = (size_t)E->n[b] * E->n[b] * E->n[b];
-        cudaError_t e = E->esize == 8
-                            ? launch_cfl<double>(cplanes<double>(u[b], cells), cells, consts_of<double>(E->p), E->cfl + 2 * b, s)
-                            : launch_cfl<float>(cplanes<float>(u[b], cells), cells, consts_of<float>(E->p), E->cfl + 2 * b, s);
-        if (e != cudaSuccess) return cuda_fail(e, "ensemble cfl");
-    }
-    const int pairs = nsteps / 2;
-    if ((flags & GMT_RUN_GRAPH) && pairs > 0) {
-        if (!E->exec) {
-            cudaGraph_t graph;
-            GMT_CUDA(cudaStreamBeginCapture(E->cap, cudaStreamCaptureModeRelaxed));
-            cudaError_t e1 = ens_enqueue_any(E, 0, flags, E->cap);
-            cudaError_t e2 = ens_enqueue_any(E, 1, flags, E->cap);
-            cudaError_t e3 = cudaStreamEndCapture(E->cap, &graph);
-            if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
-                cudaGetLastError();
-                return cuda_fail(e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3), "ensemble capture");
-            }
-            cudaError_t e4 = cudaGraphInstantiate(&E->exec, graph, 0);
-            cudaGraphDestroy(graph);
-            if (e4 != cudaSuccess) return cuda_fail(e4, "ensemble instantiate");
+    // n steps on the lanes; a run's first step reduces the CFL maxima of the initial states, the later ones
+    // find them fused into the step before
+    auto steps = [&](int n, bool start) {
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; e == cudaSuccess && i < n; ++i) e = ens_enqueue_any(E, i & 1, flags, start && i == 0);
+        return e;
+    };
+    // A replayed pair of steps pays where launching them one by one takes longer than running them.
+    size_t zones = 0;
+    for (int n : E->n) zones += (size_t)n * n * n;
+    const int pairs = (flags & GMT_RUN_GRAPH) && zones < ENS_GRAPH_ZONES * (size_t)nb ? (nsteps - 1) / 2 : 0;
+    if (pairs > 0 && !E->exec) {   // from an odd step on: the first one runs by itself, with its CFL
+        cudaGraph_t graph;
+        GMT_CUDA(cudaStreamBeginCapture(E->cap, cudaStreamCaptureModeRelaxed));
+        cudaError_t e1 = ens_fork(E, E->cap, [&] {
+            const cudaError_t e = ens_enqueue_any(E, 1, flags, false);
+            return e != cudaSuccess ? e : ens_enqueue_any(E, 0, flags, false);
+        });
+        cudaError_t e2 = cudaStreamEndCapture(E->cap, &graph);
+        if (e1 != cudaSuccess || e2 != cudaSuccess) {
+            cudaGetLastError();
+            return cuda_fail(e1 != cudaSuccess ? e1 : e2, "ensemble capture");
         }
-        for (int i = 0; i < pairs; ++i) GMT_CUDA(cudaGraphLaunch(E->exec, s));
-    } else {
-        for (int i = 0; i < pairs; ++i) {
-            GMT_CUDA(ens_enqueue_any(E, 0, flags, s));
-            GMT_CUDA(ens_enqueue_any(E, 1, flags, s));
-        }
+        cudaError_t e3 = cudaGraphInstantiate(&E->exec, graph, 0);
+        cudaGraphDestroy(graph);
+        if (e3 != cudaSuccess) return cuda_fail(e3, "ensemble instantiate");
     }
-    if (nsteps & 1) GMT_CUDA(ens_enqueue_any(E, 0, flags, s));
+    GMT_CUDA(ens_fork(E, s, [&] { return steps(pairs > 0 ? 1 : nsteps, true); }));
+    for (int i = 0; i < pairs; ++i) GMT_CUDA(cudaGraphLaunch(E->exec, s));
+    if (pairs > 0 && 1 + 2 * pairs < nsteps) GMT_CUDA(ens_fork(E, s, [&] { return ens_enqueue_any(E, 1, flags, false); }));
     int herr = 0;
     GMT_CUDA(cudaMemcpyAsync(S.data(), E->loop, nb * sizeof(LoopState), cudaMemcpyDeviceToHost, s));
     GMT_CUDA(cudaMemcpyAsync(&herr, E->err, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -1,5 +1,6 @@
 // gmt_common.cuh -- kernel argument blocks and small device helpers shared by the kernels.
 #pragma once
+#include <climits>
 #include <type_traits>
 #include <cuda.h>   // CUtensorMap (the type only; the library does not link libcuda)
 #include <cuda_runtime.h>
@@ -38,6 +39,7 @@ template <class R> struct UnsplitArgs {
     const double* dparams; // if set: dt, ch, glm_fac, ramp of this step read from device memory
     R* fmass;              // if set: the mass fluxes of every cell's lower x, y, z faces (3 planes),
                            // for the passive-species pass of the march scheme
+    int quad;              // the planes can be staged in 16-byte quads (stage_plane)
     int use_tma;           // tmap describes u: tiles clear of the box edges stage by TMA
     CUtensorMap tmap;      // 4-D map (x, y, z, variable) of u; box (ox+8) x (oy+4) x 1 x 9
     long long wait_cycles; // budget of each bounded wait (GMT_WAIT_CYCLES)
@@ -71,7 +73,7 @@ template <class R> __device__ __forceinline__ StepVals<R> step_vals(const Unspli
     return V;
 }
 
-// cp.async 4-byte global -> shared copy (L1-allocating), plus group commit / wait.
+// cp.async global -> shared copies of 4, 8 (L1-allocating) and 16 bytes, plus group commit / wait.
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));
@@ -79,6 +81,10 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }

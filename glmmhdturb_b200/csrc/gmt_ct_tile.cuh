@@ -66,19 +66,41 @@ template <class R> __host__ __device__ inline size_t ct_tile_smem_bytes(int ox, 
 // stage plane kp: the conserved cell variables, the three face fields at kp and bzf at kp+1, on
 // the region x0-2..x0+OX+2, y0-2..y0+OY+2.  SG rows have the pitch SW = OX + 8 and the region
 // starts at column 2: the layout of the TMA box (x0-4, y0-2) of (OX+8) x (OY+5) cells.
-template <class R>
-__device__ __forceinline__ void ct_stage_plane(R* __restrict__ SG, const CPlanes8<R>& q, int PN5, int PW5, int SW,
-                                               int SN5, int x0, int y0, int kp, int nx, int ny, int nz, int tid,
+// ROWS, al16: as stage_plane of the GLM tile march.
+template <bool ROWS, class R>
+__device__ __forceinline__ void ct_stage_plane(R* __restrict__ SG, const CPlanes8<R>& q, bool al16, int PN5, int PW5,
+                                               int SW, int SN5, int x0, int y0, int kp, int nx, int ny, int nz, int tid,
                                                int nt) {
-    const size_t gz = (size_t)wrapi(kp, nz), gz1 = (size_t)wrapi(kp + 1, nz);
-    for (int c = tid; c < PN5; c += nt) {
-        const int lx = c % PW5, ly = c / PW5;
-        const size_t gxy = (size_t)wrapi(x0 - 2 + lx, nx) + (size_t)nx * wrapi(y0 - 2 + ly, ny);
-        const size_t g = gxy + (size_t)nx * ny * gz, g1 = gxy + (size_t)nx * ny * gz1;
-        const int cs = ly * SW + lx + 2;
+    constexpr int Q = 16 / (int)sizeof(R);
+    const size_t nxy = (size_t)nx * ny, plane = nxy * wrapi(kp, nz), plane1 = nxy * wrapi(kp + 1, nz);
+    if (ROWS || al16) {
+        const int qw = SW / Q, jobs = qw * (SN5 / SW);
+        for (int j = tid; j < jobs; j += nt) {
+            const int row = j / qw, col = (j % qw) * Q;
+            const size_t gxy = (size_t)wrapi(x0 - 4 + col, nx) + (size_t)nx * wrapi(y0 - 2 + row, ny);
+            const int cs = row * SW + col;
+            if (al16) {
 #pragma unroll
-        for (int v = 0; v < 8; ++v) cp_async_r(SG + v * SN5 + cs, q.p[v] + g);
-        cp_async_r(SG + 8 * SN5 + cs, q.p[7] + g1);
+                for (int v = 0; v < 8; ++v) cp_async16(SG + v * SN5 + cs, q.p[v] + plane + gxy);
+                cp_async16(SG + 8 * SN5 + cs, q.p[7] + plane1 + gxy);
+            } else {
+#pragma unroll 1
+                for (int i = 0; i < Q; ++i) {
+#pragma unroll
+                    for (int v = 0; v < 8; ++v) cp_async_r(SG + v * SN5 + cs + i, q.p[v] + plane + gxy + i);
+                    cp_async_r(SG + 8 * SN5 + cs + i, q.p[7] + plane1 + gxy + i);
+                }
+            }
+        }
+    } else {
+        for (int c = tid; c < PN5; c += nt) {
+            const int lx = c % PW5, ly = c / PW5;
+            const size_t gxy = (size_t)wrapi(x0 - 2 + lx, nx) + (size_t)nx * wrapi(y0 - 2 + ly, ny);
+            const int cs = ly * SW + lx + 2;
+#pragma unroll
+            for (int v = 0; v < 8; ++v) cp_async_r(SG + v * SN5 + cs, q.p[v] + plane + gxy);
+            cp_async_r(SG + 8 * SN5 + cs, q.p[7] + plane1 + gxy);
+        }
     }
     cp_async_commit();
 }
@@ -167,7 +189,8 @@ __device__ __forceinline__ Q9<R> ct_flux(const Q9<R>& L, const Q9<R>& Rr, const 
                                          : hll_x(Lr, Rrr, K.gamma, bn, R(0), R(0)));
 }
 
-template <class R, int RECON, int RIEM, int TOX, int TOY>
+// OVER: the tile may overhang the box; the columns beyond it march on periodic images and write nothing
+template <class R, int RECON, int RIEM, int TOX, int TOY, bool OVER>
 __device__ __forceinline__ void ct_tile(const CTArgs<R>& A, int bx, int by, int bz, unsigned char* smem_raw) {
     const int OX = TOX > 0 ? TOX : A.ox, OY = TOY > 0 ? TOY : A.oy;
     const int PW = OX + 4, PN = lay_n<R>((OX + 4) * (OY + 4));   // padded array lengths (Lay layout)
@@ -214,27 +237,42 @@ __device__ __forceinline__ void ct_tile(const CTArgs<R>& A, int bx, int by, int 
 
     if constexpr (std::is_same<R, float>::value) {
         if (A.trig8)
-            for (int i = tid; i < 2 * OX; i += NT)
+            for (int i = tid; i < 2 * (OVER ? min(OX, nx - x0) : OX); i += NT)
                 reinterpret_cast<float4*>(TS)[i] = reinterpret_cast<const float4*>(A.trig8 + 8 * (size_t)x0)[i];
     }
     uint64_t* mbar = reinterpret_cast<uint64_t*>(red + 32);
-    for (int j = 0; j < 3; ++j) {
-        ct_stage_plane(SG, A.q, PN5, PW5, SW, SN5, x0, y0, z0 - 2 + j, nx, ny, nz, tid, NT);
+    const bool quad = A.quad != 0;
+    // prologue: three planes in flight together, two staged in the states' arrays (as in the GLM tile)
+    if (36 * RN >= 18 * SN5 && ((unsigned)__cvta_generic_to_shared(ST) & 15u) == 0) {
+        for (int j = 0; j < 3; ++j)
+            ct_stage_plane<!OVER>(j == 2 ? SG : ST + j * 9 * SN5, A.q, quad, PN5, PW5, SW, SN5, x0, y0, z0 - 2 + j, nx, ny, nz, tid,
+                           NT);
         cp_async_wait_all();
         __syncthreads();
-        ct_unstage_plane(PR + mod3(z0 - 2 + j) * 9 * PN, FB + mod3(z0 - 2 + j) * 3 * PN, SG, PN, PNc, PW, SN5, SW, K,
-                         tid, NT);
-        if (j == 2 && tid == 0) {
-            mbar_init(mbar, tma ? 1u : (unsigned)NT);
-            if (tma) fence_mbar_init();
+        for (int j = 0; j < 3; ++j)
+            ct_unstage_plane(PR + mod3(z0 - 2 + j) * 9 * PN, FB + mod3(z0 - 2 + j) * 3 * PN, j == 2 ? SG : ST + j * 9 * SN5,
+                             PN, PNc, PW, SN5, SW, K, tid, NT);
+    } else {
+        for (int j = 0; j < 3; ++j) {
+            ct_stage_plane<!OVER>(SG, A.q, quad, PN5, PW5, SW, SN5, x0, y0, z0 - 2 + j, nx, ny, nz, tid, NT);
+            cp_async_wait_all();
+            __syncthreads();
+            ct_unstage_plane(PR + mod3(z0 - 2 + j) * 9 * PN, FB + mod3(z0 - 2 + j) * 3 * PN, SG, PN, PNc, PW, SN5, SW, K,
+                             tid, NT);
+            if (j < 2) __syncthreads();
         }
-        __syncthreads();
     }
+    if (tid == 0) {
+        mbar_init(mbar, tma ? 1u : (unsigned)NT);
+        if (tma) fence_mbar_init();
+    }
+    __syncthreads();
 
     Q9<R> pPz, Fzlo, Fxh, Fyh;
 #pragma unroll
     for (int v = 0; v < 9; ++v) { pPz.v[v] = R(0); Fzlo.v[v] = R(0); Fxh.v[v] = R(0); Fyh.v[v] = R(0); }
     const int gx = x0 + tx, gy = y0 + ty;
+    const int zw = !OVER || (gx < nx && gy < ny) ? z0 : INT_MAX;   // first plane this column writes
     const int cown = (tx + 2) + PW * (ty + 2);
     const int rown = (tx + 1) + RW * (ty + 1);
     const int ixh = (tx + 2) + RW * (ty + 1);
@@ -256,8 +294,8 @@ __device__ __forceinline__ void ct_tile(const CTArgs<R>& A, int bx, int by, int 
                 }
             }
             if (!tma && !A.wait_test) {
-                ct_stage_plane(SG, A.q, PN5, PW5, SW, SN5, x0, y0, kr + 2, nx, ny, nz, tid >= stg0 ? tid - stg0 : PN5,
-                               NT - stg0);
+                ct_stage_plane<!OVER>(SG, A.q, quad, PN5, PW5, SW, SN5, x0, y0, kr + 2, nx, ny, nz,
+                               tid >= stg0 ? tid - stg0 : INT_MAX, NT - stg0);
                 mbar_arrive_cp_async(mbar);
             }
         }
@@ -289,7 +327,7 @@ __device__ __forceinline__ void ct_tile(const CTArgs<R>& A, int bx, int by, int 
             if (!first) {
                 // the old cell state written out below, loaded before the z-face solve so that the
                 // solve hides its latency
-                const bool wr = kr - 1 >= z0;
+                const bool wr = kr - 1 >= zw;
                 const int kf = kr - 1;
                 const size_t g = (size_t)gx + (size_t)nx * ((size_t)gy + (size_t)ny * (wr ? kf : 0));
                 R u0[5];
@@ -381,7 +419,7 @@ __device__ __forceinline__ void ct_tile(const CTArgs<R>& A, int bx, int by, int 
         // the forcing row table of the tile's rows for plane kr, written out in the next phase
         if constexpr (std::is_same<R, float>::value) {
             if (turb && A.trig8 && kr >= z0 && kr < z1)
-                for (int i = tid; i < 6 * OY; i += NT)
+                for (int i = tid; i < 6 * (OVER ? min(OY, ny - y0) : OY); i += NT)
                     reinterpret_cast<float4*>(BS)[i] =
                         reinterpret_cast<const float4*>(A.btab + ((size_t)kr * ny + y0) * 24)[i];
         }
@@ -396,10 +434,10 @@ __device__ __forceinline__ void ct_tile(const CTArgs<R>& A, int bx, int by, int 
     if (tid == 0) mbar_inval(mbar);
 }
 
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0, bool OVER = TOX == 0>
 __global__ void __launch_bounds__(MAXT, MINB) ct_tile_kernel(const __grid_constant__ CTArgs<R> A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    ct_tile<R, RECON, RIEM, TOX, TOY>(A, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
+    ct_tile<R, RECON, RIEM, TOX, TOY, OVER>(A, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
 }
 
 template <class R> __device__ __forceinline__ R ct_upwind(R flux, R minus, R plus) {
@@ -620,9 +658,9 @@ template <class R> inline bool ct_quad_ok(const CTArgs<R>& A) {
 }
 
 // launch: pass A (tile kernel), then B1 and B2; nt <= 0 in A configures the kernel only
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
-static cudaError_t ct_go(const CTArgs<R>& A, cudaStream_t s, bool configure_only) {
-    auto k = ct_tile_kernel<R, RECON, RIEM, MAXT, MINB, TOX, TOY>;
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX, int TOY, bool OVER>
+static cudaError_t ct_run_tile(const CTArgs<R>& A, cudaStream_t s, bool configure_only) {
+    auto k = ct_tile_kernel<R, RECON, RIEM, MAXT, MINB, TOX, TOY, OVER>;
     static int configured[64] = {0};
     {
         cudaError_t e = configure_once(k, configured);
@@ -631,8 +669,21 @@ static cudaError_t ct_go(const CTArgs<R>& A, cudaStream_t s, bool configure_only
     if (configure_only) return cudaSuccess;
     const int nt = A.ox * A.oy;
     if (nt > MAXT || nt < 1) return cudaErrorInvalidConfiguration;
-    dim3 grid(A.nx / A.ox, A.ny / A.oy, (A.nz + A.lz - 1) / A.lz);
+    dim3 grid((A.nx + A.ox - 1) / A.ox, (A.ny + A.oy - 1) / A.oy, (A.nz + A.lz - 1) / A.lz);
     k<<<grid, nt, ct_tile_smem_bytes<R>(A.ox, A.oy), s>>>(A);
+    return cudaGetLastError();
+}
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
+static cudaError_t ct_go(const CTArgs<R>& A, cudaStream_t s, bool configure_only) {
+    if (configure_only) {
+        cudaError_t e = ct_run_tile<R, RECON, RIEM, MAXT, MINB, TOX, TOY, true>(A, s, true);
+        if (e == cudaSuccess && TOX > 0) e = ct_run_tile<R, RECON, RIEM, MAXT, MINB, TOX, TOY, TOX == 0>(A, s, true);
+        return e;
+    }
+    const bool over = TOX == 0 || A.nx % A.ox != 0 || A.ny % A.oy != 0;
+    cudaError_t e = over ? ct_run_tile<R, RECON, RIEM, MAXT, MINB, TOX, TOY, true>(A, s, false)
+                         : ct_run_tile<R, RECON, RIEM, MAXT, MINB, TOX, TOY, TOX == 0>(A, s, false);
+    if (e != cudaSuccess) return e;
     const size_t n = (size_t)A.nx * A.ny * A.nz;
     if constexpr (std::is_same<R, float>::value) {
         if (ct_quad_ok(A)) {

@@ -17,13 +17,6 @@ cudaError_t launch_unsplit(const UnsplitArgs<double>& A, int recon, int riem, cu
 int unsplit_max_threads(int dtype_bytes);
 cudaError_t unsplit_prepare_f32();   // shared-memory attributes of every step kernel
 cudaError_t unsplit_prepare_f64();
-struct EnsItem;
-// tile of the ensemble kernel: ens_tile_x<R>() columns by 16 rows (32 in FP32, 16 in FP64)
-template <class R> constexpr int ens_tile_x() { return sizeof(R) == 4 ? 32 : 16; }
-cudaError_t launch_ensemble(const UnsplitArgs<float>* boxes, const EnsItem* items, int nitems, unsigned* queue,
-                            int recon, int riem, int nsm, cudaStream_t s);
-cudaError_t launch_ensemble(const UnsplitArgs<double>* boxes, const EnsItem* items, int nitems, unsigned* queue,
-                            int recon, int riem, int nsm, cudaStream_t s);
 size_t unsplit_smem(int dtype_bytes, int ox, int oy);
 // tiled march (the unsplit tile with the march scheme; no passive species)
 cudaError_t launch_march_tiled(const UnsplitArgs<float>& A, int recon, cudaStream_t s);
@@ -62,6 +55,7 @@ template <class R> struct CTArgs {
     const R* trig8;        // FP32 or null: x table of 2 cos, -2 sin (force_accel_f32)
     R* scratch;            // 15 planes: lower-face EMF data and cell EMFs (12), edge EMFs (3)
     int* err;              // device flag set when a bounded wait gives up
+    int quad;              // the planes can be staged in 16-byte quads
     int use_tma;           // tmap8/tmap1 describe q: tiles clear of the box edges stage by TMA
     CUtensorMap tmap8;     // 4-D map (x, y, z, variable) of q, box (ox+8) x (oy+5) x 1 x 8
     CUtensorMap tmap1;     // the same tensor, box (ox+8) x (oy+5) x 1 x 1 (bzf of the next plane)

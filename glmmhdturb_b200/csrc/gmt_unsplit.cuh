@@ -155,17 +155,42 @@ __device__ __forceinline__ int mod3(int k) {
 // The staging plane SG holds the conserved variables of the ring region (x0-2.., y0-2..) with a
 // row pitch SW = OX + 8 and the region starting at column 2: exactly the box (x0-4, y0-2) of
 // (OX+8) x (OY+4) cells that one TMA copy delivers (its first column 16-byte aligned).
-template <class R>
-__device__ __forceinline__ void stage_plane(R* __restrict__ SG, const CPlanes<R>& u, int PN, int PW, int SW, int SN,
-                                            int x0, int y0, int kp, int nx, int ny, int nz, int tid, int nt) {
-    const int gz = wrapi(kp, nz);
-    for (int c = tid; c < PN; c += nt) {
-        int lx = c % PW, ly = c / PW;
-        int gx = wrapi(x0 - 2 + lx, nx), gy = wrapi(y0 - 2 + ly, ny);
-        size_t g = (size_t)gx + (size_t)nx * ((size_t)gy + (size_t)ny * gz);
-        const int cs = ly * SW + lx + 2;
+// Rows of whole quads (nx and the tile width multiples of 4, in FP64 of 2): a quad of 16 bytes never
+// straddles the periodic boundary, so the staged rows are copied quad by quad -- one 16-byte copy each,
+// or, where a plane is not 16-byte aligned (al16 false), one copy per cell.  A 4-byte copy per cell costs
+// every thread of a 32x16 tile 15 copies and their address arithmetic per plane, 4 % of the step's
+// instructions.  ROWS: the tile divides the box, so its rows are known to be whole quads and the
+// cell-by-cell loop for other rows is not compiled in (it took registers from the 128-register tiles
+// that never run it; 512^3: 11.28 ms against 11.10 ms).
+template <bool ROWS, class R>
+__device__ __forceinline__ void stage_plane(R* __restrict__ SG, const CPlanes<R>& u, bool al16, int PN, int PW, int SW,
+                                            int SN, int x0, int y0, int kp, int nx, int ny, int nz, int tid, int nt) {
+    constexpr int Q = 16 / (int)sizeof(R);
+    const size_t plane = (size_t)nx * ny * wrapi(kp, nz);
+    if (ROWS || al16) {
+        const int qw = SW / Q, jobs = qw * (SN / SW);
+        for (int j = tid; j < jobs; j += nt) {
+            const int row = j / qw, col = (j % qw) * Q;
+            const size_t g = plane + (size_t)wrapi(x0 - 4 + col, nx) + (size_t)nx * wrapi(y0 - 2 + row, ny);
+            const int cs = row * SW + col;
+            if (al16) {
 #pragma unroll
-        for (int v = 0; v < 9; ++v) cp_async_r(SG + v * SN + cs, u.p[v] + g);
+                for (int v = 0; v < 9; ++v) cp_async16(SG + v * SN + cs, u.p[v] + g);
+            } else {
+#pragma unroll 1
+                for (int i = 0; i < Q; ++i)
+#pragma unroll
+                    for (int v = 0; v < 9; ++v) cp_async_r(SG + v * SN + cs + i, u.p[v] + g + i);
+            }
+        }
+    } else {
+        for (int c = tid; c < PN; c += nt) {
+            const int lx = c % PW, ly = c / PW;
+            const size_t g = plane + (size_t)wrapi(x0 - 2 + lx, nx) + (size_t)nx * wrapi(y0 - 2 + ly, ny);
+            const int cs = ly * SW + lx + 2;
+#pragma unroll
+            for (int v = 0; v < 9; ++v) cp_async_r(SG + v * SN + cs, u.p[v] + g);
+        }
     }
     cp_async_commit();
 }
@@ -185,8 +210,8 @@ __device__ __forceinline__ void unstage_plane(R* __restrict__ PRs, const R* __re
 }
 
 // shared-memory layout of the tile march: PR ring, ST states, then (128-byte aligned, as a TMA
-// destination) the staging plane SG, then (16-byte aligned) the reduction and mbarrier words and,
-// in FP32, the tile's forcing tables (8 floats per column, 24 per row)
+// destination) the staging plane SG, then (16-byte aligned) the reduction and mbarrier words, and, in
+// FP32, the tile's forcing tables (8 floats per column, 24 per row)
 template <class R> __host__ __device__ inline size_t unsplit_sg_offset(int ox, int oy) {
     size_t PN = (size_t)lay_n<R>((ox + 4) * (oy + 4)), RN = (size_t)lay_n<R>((ox + 2) * (oy + 2));
     return ((27 * PN + 36 * RN) * sizeof(R) + 127) / 128 * 128;
@@ -310,11 +335,13 @@ template <class R, int RECON> struct MarchScheme {
 };
 
 // One tile (bx, by) x z-chunk bz of one box.  TOX, TOY > 0 fix the tile at compile time
-// (constant shared-memory offsets); 0 = runtime tile.  Used by the single-box kernel (one tile per
-// block) and by the ensemble kernel (a queue of tiles over many boxes).
-// TMA: the kernel's A is a grid-constant parameter, so A.tmap can be handed to the TMA unit
-// (the ensemble kernel copies its arguments from global memory and keeps the cp.async path).
-template <class R, class S, int TOX, int TOY, bool OVERHANG = false, bool TMA = false>
+// (constant shared-memory offsets); 0 = runtime tile.  A is the kernel's grid-constant parameter, so
+// A.tmap can be handed to the TMA unit.
+// OVER: the tile may overhang the box (a box width or height that is no multiple of the tile).  The
+// columns beyond the box march along on periodic images of the row's first cells, so every neighbour
+// sees the values it would see anyway; their writes (and CFL maxima) are left out.  A kernel of its
+// own, since the test costs the 128-register production tile 3 % in spills (512^3: 11.2 -> 11.6 ms).
+template <class R, class S, int TOX, int TOY, bool OVER>
 __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepVals<R>& V, int bx, int by, int bz,
                                             unsigned char* smem_raw) {
     const int OX = TOX > 0 ? TOX : A.ox, OY = TOY > 0 ? TOY : A.oy;
@@ -351,35 +378,44 @@ __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepV
 
     // a tile whose staged region (x0-4 .. x0+OX+3, y0-2 .. y0+OY+1) lies inside the box stages its
     // planes by one TMA copy each (the tensor map addresses no periodic images); the others, and
-    // every tile when the caller supplied no map, by per-thread cp.async
-    bool tma = false;
-    if constexpr (TMA) {
-        tma = A.use_tma && !A.wait_test && x0 >= 4 && x0 + OX + 4 <= nx && y0 >= 2 && y0 + OY + 2 <= ny;
-        // a TMA destination must be 128-byte aligned; otherwise stay on cp.async
-        if ((unsigned)__cvta_generic_to_shared(SG) & 127u) tma = false;
-    }
+    // every tile when the caller supplied no map, by per-thread cp.async (not by untiled bulk copies of
+    // the rows: 180 of 160 bytes a plane took longer than the plane, 64^3 89 us against 40)
+    bool tma = A.use_tma && !A.wait_test && x0 >= 4 && x0 + OX + 4 <= nx && y0 >= 2 && y0 + OY + 2 <= ny;
+    // a TMA destination must be 128-byte aligned; otherwise stay on cp.async
+    if ((unsigned)__cvta_generic_to_shared(SG) & 127u) tma = false;
     const unsigned tma_bytes = (unsigned)(9 * SN * sizeof(R));
 
-    // (the ensemble kernel, OVERHANG, keeps the tables in global memory: staged there it measured
-    // 2 % slower, its 128 registers already spilling)
-    if constexpr (std::is_same<R, float>::value && !OVERHANG) {
+    if constexpr (std::is_same<R, float>::value) {
         if (A.trig8)
-            for (int i = tid; i < 2 * OX; i += NT)
+            for (int i = tid; i < 2 * (OVER ? min(OX, nx - x0) : OX); i += NT)
                 reinterpret_cast<float4*>(TS)[i] = reinterpret_cast<const float4*>(A.trig8 + 8 * (size_t)x0)[i];
     }
-    // prologue: primitives of planes z0-2, z0-1, z0
+    const bool quad = A.quad != 0;
     uint64_t* mbar = reinterpret_cast<uint64_t*>(red + 32);
-    for (int j = 0; j < 3; ++j) {
-        stage_plane(SG, A.u, PNc, PW, SW, SN, x0, y0, z0 - 2 + j, nx, ny, nz, tid, NT);
+    // prologue: primitives of planes z0-2, z0-1, z0.  The states' arrays are still free, so all three
+    // planes are in flight together, two of them staged there (where they fit, aligned).
+    if (36 * RN >= 18 * SN && ((unsigned)__cvta_generic_to_shared(ST) & 15u) == 0) {
+        for (int j = 0; j < 3; ++j)
+            stage_plane<!OVER>(j == 2 ? SG : ST + j * 9 * SN, A.u, quad, PNc, PW, SW, SN, x0, y0, z0 - 2 + j, nx, ny, nz, tid, NT);
         cp_async_wait_all();
         __syncthreads();
-        unstage_plane(PR + mod3(z0 - 2 + j) * 9 * PN, SG, PN, PNc, PW, SW, SN, K, S::prim_floor(K), tid, NT);
-        if (j == 2 && tid == 0) {
-            mbar_init(mbar, tma ? 1u : (unsigned)NT);
-            if (tma) fence_mbar_init();
+        for (int j = 0; j < 3; ++j)
+            unstage_plane(PR + mod3(z0 - 2 + j) * 9 * PN, j == 2 ? SG : ST + j * 9 * SN, PN, PNc, PW, SW, SN, K,
+                          S::prim_floor(K), tid, NT);
+    } else {
+        for (int j = 0; j < 3; ++j) {
+            stage_plane<!OVER>(SG, A.u, quad, PNc, PW, SW, SN, x0, y0, z0 - 2 + j, nx, ny, nz, tid, NT);
+            cp_async_wait_all();
+            __syncthreads();
+            unstage_plane(PR + mod3(z0 - 2 + j) * 9 * PN, SG, PN, PNc, PW, SW, SN, K, S::prim_floor(K), tid, NT);
+            if (j < 2) __syncthreads();
         }
-        __syncthreads();
     }
+    if (tid == 0) {
+        mbar_init(mbar, tma ? 1u : (unsigned)NT);
+        if (tma) fence_mbar_init();
+    }
+    __syncthreads();
 
     // registers carried along the column: +z state of the previous plane, F_z at its lower face,
     // and this thread's own x/y face fluxes of the previous plane
@@ -388,14 +424,8 @@ __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepV
     for (int v = 0; v < 9; ++v) { pPz.v[v] = R(0); Fzlo.v[v] = R(0); Fxh.v[v] = R(0); Fyh.v[v] = R(0); }
     R cmax = R(0), smax = R(0);   // exact maxima in R, widened to FP64 once per block
     double damp = 0.0;            // record mode: this thread's share of dL/d(forcing amplitude)
-    // OVERHANG: a tile may overhang the box (an ensemble box narrower than a tile multiple); the
-    // overhanging columns recompute the periodic images of cells at the start of the row, bit for
-    // bit the same values, so their duplicate writes (and CFL maxima) are harmless
-    int gx = x0 + tx, gy = y0 + ty;
-    if (OVERHANG) {
-        gx = gx < nx ? gx : gx - nx;
-        gy = gy < ny ? gy : gy - ny;
-    }
+    const int gx = x0 + tx, gy = y0 + ty;
+    const int zw = !OVER || (gx < nx && gy < ny) ? z0 : INT_MAX;   // first plane this column writes
     const int cown = (tx + 2) + PW * (ty + 2);     // ring-local index of the owned cell
     const int rown = (tx + 1) + RW * (ty + 1);     // recon-local index of the owned cell
     const int ixh = (tx + 2) + RW * (ty + 1);      // slot of the +x neighbour
@@ -411,18 +441,14 @@ __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepV
         const bool load = kr + 2 <= z1 + 1;
         const int s0 = mod3(kr), sm = mod3(kr - 1), sp = mod3(kr + 1);
         if (load) {
-            if constexpr (TMA) {
-                if (tma) {
-                    if (tid == 0) {
-                        fence_proxy_async_smem();   // the previous plane's reads of SG come first
-                        mbar_arrive_expect_tx(mbar, tma_bytes);
-                        tma_load_4d(SG, &A.tmap, x0 - 4, y0 - 2, wrapi(kr + 2, nz), 0, mbar);
-                    }
-                }
+            if (tma && tid == 0) {
+                fence_proxy_async_smem();   // the previous plane's reads of SG come first
+                mbar_arrive_expect_tx(mbar, tma_bytes);
+                tma_load_4d(SG, &A.tmap, x0 - 4, y0 - 2, wrapi(kr + 2, nz), 0, mbar);
             }
             if (!tma && !A.wait_test) {
-                stage_plane(SG, A.u, PNc, PW, SW, SN, x0, y0, kr + 2, nx, ny, nz, tid >= stg0 ? tid - stg0 : PNc,
-                            NT - stg0);
+                stage_plane<!OVER>(SG, A.u, quad, PNc, PW, SW, SN, x0, y0, kr + 2, nx, ny, nz,
+                                   tid >= stg0 ? tid - stg0 : INT_MAX, NT - stg0);
                 mbar_arrive_cp_async(mbar);
             }
         }
@@ -445,7 +471,7 @@ __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepV
             const size_t ncell = (size_t)nx * ny * nz;
             auto record = [&](int k, const Q9<R>& f) {
                 if constexpr (S::kRecord) {
-                    if (kr >= z0 && kr < z1)
+                    if (kr >= zw && kr < z1)
                         rec_put(A, ncell, k, (size_t)gx + (size_t)nx * ((size_t)gy + (size_t)ny * (size_t)kr), f);
                 }
             };
@@ -478,13 +504,12 @@ __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepV
             if (!first && !last) record(4, Pz);
             if (!first) {
                 // the old state of the cell written out below, loaded before the z-face solve so that
-                // the solve hides its latency (S::kEarlyOld), else at the write-out; the ensemble
-                // kernel (OVERHANG) measured 7 % slower with the early load
-                const bool wr = kr - 1 >= z0;
+                // the solve hides its latency (S::kEarlyOld), else at the write-out
+                const bool wr = kr - 1 >= zw;
                 const int kf = kr - 1;
                 const size_t g = (size_t)gx + (size_t)nx * ((size_t)gy + (size_t)ny * (wr ? kf : 0));
                 Q9<R> u0;
-                if constexpr (S::kEarlyOld && !OVERHANG) {
+                if constexpr (S::kEarlyOld) {
 #pragma unroll
                     for (int v = 0; v < 9; ++v) u0.v[v] = wr ? __ldg(A.u.p[v] + g) : R(0);
                 }
@@ -495,10 +520,10 @@ __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepV
                     Q9<R> q;
 #pragma unroll
                     for (int v = 0; v < 9; ++v)
-                        q.v[v] = ((S::kEarlyOld && !OVERHANG) ? u0.v[v] : A.u.p[v][g]) + dtdx * (XY.v[v] + (Fzlo.v[v] - Fzhi.v[v]));
+                        q.v[v] = (S::kEarlyOld ? u0.v[v] : A.u.p[v][g]) + dtdx * (XY.v[v] + (Fzlo.v[v] - Fzhi.v[v]));
                     R ax = R(0), ay = R(0), az = R(0);
                     if (turb) {
-                        if constexpr (std::is_same<R, float>::value && !OVERHANG) {
+                        if constexpr (std::is_same<R, float>::value) {
                             if (A.trig8) force_accel_f32(BS + 24 * ty, TS, tx, V.ramp, ax, ay, az);
                             else force_accel(A.btab + ((size_t)kf * ny + gy) * 24, A.trigx, nx, gx, V.ramp, ax, ay, az);
                         } else {
@@ -593,9 +618,9 @@ __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepV
             }
         }
         // the forcing row table of the tile's rows for plane kr, written out in the next phase R
-        if constexpr (std::is_same<R, float>::value && !OVERHANG) {
+        if constexpr (std::is_same<R, float>::value) {
             if (turb && A.trig8 && kr >= z0 && kr < z1)
-                for (int i = tid; i < 6 * OY; i += NT)
+                for (int i = tid; i < 6 * (OVER ? min(OY, ny - y0) : OY); i += NT)
                     reinterpret_cast<float4*>(BS)[i] =
                         reinterpret_cast<const float4*>(A.btab + ((size_t)kr * ny + y0) * 24)[i];
         }
@@ -630,48 +655,19 @@ __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepV
     }
 }
 
-template <class R, int RECON, int RIEM, int TOX, int TOY, bool OVERHANG = false, bool TMA = false>
-__device__ __forceinline__ void unsplit_tile(const UnsplitArgs<R>& A, const StepVals<R>& V, int bx, int by, int bz,
-                                             unsigned char* smem_raw) {
-    scheme_tile<R, UnsplitScheme<R, RECON, RIEM>, TOX, TOY, OVERHANG, TMA>(A, V, bx, by, bz, smem_raw);
-}
-
-// A tile = (box, bx, by, bz) work item of the ensemble kernel.
-struct EnsItem { int box, bx, by, bz; };
-
-// Persistent ensemble step: each block takes work items from a global queue (one atomic per
-// item) until the queue is drained; every box has its own arguments, step values and CFL slot.
-template <class R, int RECON, int RIEM, int TOX, int TOY, int MAXT, int MINB>
-__global__ void __launch_bounds__(MAXT, MINB) ensemble_kernel(const UnsplitArgs<R>* __restrict__ boxes,
-                                                              const EnsItem* __restrict__ items, int nitems,
-                                                              unsigned* queue) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ int item_s;
-    for (;;) {
-        if (threadIdx.x == 0) item_s = (int)atomicAdd(queue, 1u);
-        __syncthreads();
-        const int it = item_s;
-        __syncthreads();
-        if (it >= nitems) break;
-        const EnsItem w = items[it];
-        const UnsplitArgs<R> A = boxes[w.box];
-        unsplit_tile<R, RECON, RIEM, TOX, TOY, true>(A, step_vals(A), w.bx, w.by, w.bz, smem_raw);
-        __syncthreads();
-    }
-}
-
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
+// TOX = 0 (a runtime tile) always allows for overhang
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0, bool OVER = TOX == 0>
 __global__ void __launch_bounds__(MAXT, MINB) unsplit_kernel(const __grid_constant__ UnsplitArgs<R> A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    unsplit_tile<R, RECON, RIEM, TOX, TOY, false, true>(A, step_vals(A), blockIdx.x, blockIdx.y,
-                                                                                 blockIdx.z, smem_raw);
+    scheme_tile<R, UnsplitScheme<R, RECON, RIEM>, TOX, TOY, OVER>(A, step_vals(A), blockIdx.x, blockIdx.y,
+                                                                                blockIdx.z, smem_raw);
 }
 
 // Tiled march step (the scheme behind march_run_dev); RECON is RECON_MC or RECON_PPM.
-template <class R, int RECON, int MAXT, int MINB, int TOX = 0, int TOY = 0>
+template <class R, int RECON, int MAXT, int MINB, int TOX = 0, int TOY = 0, bool OVER = TOX == 0>
 __global__ void __launch_bounds__(MAXT, MINB) march_tile_kernel(const __grid_constant__ UnsplitArgs<R> A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    scheme_tile<R, MarchScheme<R, RECON>, TOX, TOY, false, true>(
+    scheme_tile<R, MarchScheme<R, RECON>, TOX, TOY, OVER>(
         A, step_vals(A), blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
 }
 

@@ -29,30 +29,33 @@ template <class K> static cudaError_t configure_once(K k, int* configured) {
     return cudaSuccess;
 }
 
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0> struct UnsplitCfg {
-    static int configured[64];
-};
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX, int TOY>
-int UnsplitCfg<R, RECON, RIEM, MAXT, MINB, TOX, TOY>::configured[64] = {0};
-
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
-static cudaError_t unsplit_configure() {
-    return configure_once(unsplit_kernel<R, RECON, RIEM, MAXT, MINB, TOX, TOY>,
-                          UnsplitCfg<R, RECON, RIEM, MAXT, MINB, TOX, TOY>::configured);
-}
-
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
-static cudaError_t unsplit_go(const UnsplitArgs<R>& A, cudaStream_t s) {
-    auto k = unsplit_kernel<R, RECON, RIEM, MAXT, MINB, TOX, TOY>;
+// one kernel; configure_only sets its attributes
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX, int TOY, bool OVER>
+static cudaError_t unsplit_run(const UnsplitArgs<R>* A, cudaStream_t s, bool configure_only) {
+    auto k = unsplit_kernel<R, RECON, RIEM, MAXT, MINB, TOX, TOY, OVER>;
+    static int configured[64] = {0};
     {
-        cudaError_t e = unsplit_configure<R, RECON, RIEM, MAXT, MINB, TOX, TOY>();
+        cudaError_t e = configure_once(k, configured);
         if (e != cudaSuccess) return e;
     }
-    const int nt = A.ox * A.oy;
+    if (configure_only) return cudaSuccess;
+    const int nt = A->ox * A->oy;
     if (nt > MAXT || nt < 1) return cudaErrorInvalidConfiguration;
-    dim3 grid(A.nx / A.ox, A.ny / A.oy, (A.nz + A.lz - 1) / A.lz);
-    k<<<grid, nt, unsplit_smem_bytes<R>(A.ox, A.oy), s>>>(A);
+    dim3 grid((A->nx + A->ox - 1) / A->ox, (A->ny + A->oy - 1) / A->oy, (A->nz + A->lz - 1) / A->lz);
+    k<<<grid, nt, unsplit_smem_bytes<R>(A->ox, A->oy), s>>>(*A);
     return cudaGetLastError();
+}
+template <class R> inline bool overhangs(const UnsplitArgs<R>& A) { return A.nx % A.ox != 0 || A.ny % A.oy != 0; }
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
+static cudaError_t unsplit_configure() {
+    cudaError_t e = unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, true>(nullptr, 0, true);
+    if (e == cudaSuccess && TOX > 0) e = unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, TOX == 0>(nullptr, 0, true);
+    return e;
+}
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
+static cudaError_t unsplit_go(const UnsplitArgs<R>& A, cudaStream_t s) {
+    if (TOX == 0 || overhangs(A)) return unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, true>(&A, s, false);
+    return unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, TOX == 0>(&A, s, false);
 }
 
 template <class R, int MAXT, int MINB>
@@ -92,32 +95,11 @@ template <class R, int MAXT, int MINB> static int unsplit_regs_of_t(int recon, i
 }  // namespace gmt
 
 namespace gmt {
-// ensemble launcher: persistent grid, one (FP32) or two (FP64) blocks per SM
-template <class R, int RECON, int RIEM>
-static cudaError_t ensemble_go(const UnsplitArgs<R>* boxes, const EnsItem* items, int nitems, unsigned* queue,
-                               int nsm, cudaStream_t s) {
-    // FP32: 32x16 tiles, 512 threads, one block per SM; FP64: 16x16 tiles, 256 threads
-    constexpr bool F32 = sizeof(R) == 4;
-    constexpr int OX = ens_tile_x<R>(), OY = 16, NT = OX * OY, MB = F32 ? 1 : 2;
-    auto k = ensemble_kernel<R, RECON, RIEM, OX, OY, NT, MB>;
-    static int configured[64] = {0};
-    {
-        cudaError_t e = configure_once(k, configured);
-        if (e != cudaSuccess) return e;
-    }
-    if (nitems <= 0) return cudaSuccess;   // configure only
-    int nb = std::max(1, std::min(nitems, MB * nsm));
-    k<<<nb, NT, unsplit_smem_bytes<R>(OX, OY), s>>>(boxes, items, nitems, queue);
-    return cudaGetLastError();
-}
-}  // namespace gmt
-
-namespace gmt {
 // tiled march launcher (recon MC or PPM; the march has no minmod variant, spike_mhd.cu:118-123);
 // nt <= 0 configures the kernel only
-template <class R, int RECON, int MAXT, int MINB, int TOX = 0, int TOY = 0>
-static cudaError_t march_go(const UnsplitArgs<R>& A, cudaStream_t s, bool configure_only) {
-    auto k = march_tile_kernel<R, RECON, MAXT, MINB, TOX, TOY>;
+template <class R, int RECON, int MAXT, int MINB, int TOX, int TOY, bool OVER>
+static cudaError_t march_run(const UnsplitArgs<R>& A, cudaStream_t s, bool configure_only) {
+    auto k = march_tile_kernel<R, RECON, MAXT, MINB, TOX, TOY, OVER>;
     static int configured[64] = {0};
     {
         cudaError_t e = configure_once(k, configured);
@@ -126,9 +108,19 @@ static cudaError_t march_go(const UnsplitArgs<R>& A, cudaStream_t s, bool config
     if (configure_only) return cudaSuccess;
     const int nt = A.ox * A.oy;
     if (nt > MAXT || nt < 1) return cudaErrorInvalidConfiguration;
-    dim3 grid(A.nx / A.ox, A.ny / A.oy, (A.nz + A.lz - 1) / A.lz);
+    dim3 grid((A.nx + A.ox - 1) / A.ox, (A.ny + A.oy - 1) / A.oy, (A.nz + A.lz - 1) / A.lz);
     k<<<grid, nt, unsplit_smem_bytes<R>(A.ox, A.oy), s>>>(A);
     return cudaGetLastError();
+}
+template <class R, int RECON, int MAXT, int MINB, int TOX = 0, int TOY = 0>
+static cudaError_t march_go(const UnsplitArgs<R>& A, cudaStream_t s, bool configure_only) {
+    if (configure_only) {
+        cudaError_t e = march_run<R, RECON, MAXT, MINB, TOX, TOY, true>(A, s, true);
+        if (e == cudaSuccess && TOX > 0) e = march_run<R, RECON, MAXT, MINB, TOX, TOY, TOX == 0>(A, s, true);
+        return e;
+    }
+    if (TOX == 0 || overhangs(A)) return march_run<R, RECON, MAXT, MINB, TOX, TOY, true>(A, s, false);
+    return march_run<R, RECON, MAXT, MINB, TOX, TOY, TOX == 0>(A, s, false);
 }
 template <class R, int MAXT, int MINB>
 static cudaError_t march_dispatch_t(const UnsplitArgs<R>& A, int recon, cudaStream_t s, bool configure_only) {

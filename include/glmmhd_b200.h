@@ -136,11 +136,11 @@ enum { GMT_RUN_CH_MAXSIGNAL = 1, GMT_RUN_FORCING = 2, GMT_RUN_GRAPH = 4 };
 int gmt_run(gmt_ctx* ctx, void* u, void* w, int32_t nsteps, double t0, double t_end, int32_t flags, void* stream,
             double* t_out, int32_t* which);
 
-/* --- batched ensemble: many periodic boxes of different sizes in one persistent launch per step -
+/* --- batched ensemble: many periodic boxes of different sizes advanced together
  * (no counterpart in the reference).  Every box: its own n^3 grid (n a multiple of 16), forcing
- * amplitude and seed; the physics of `base`.  Each step: one tick per box, the conditional forcing
- * updates, and one persistent kernel over a queue of tile work items of all boxes (32x16 columns
- * in FP32, 16x16 in FP64, z-chunks of at most 64 planes). */
+ * amplitude and seed; the physics of `base`.  Each box advances on a stream of its own, forked from
+ * the caller's: a tick, the conditional forcing update and its step kernel per step, ordered only
+ * after the box's own previous step, so the boxes fill the chip together. */
 typedef struct gmt_ensemble gmt_ensemble;
 int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, const double* turb_amp,
                         const uint32_t* seeds, gmt_ensemble** out);
