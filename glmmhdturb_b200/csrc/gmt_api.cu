@@ -69,12 +69,24 @@ double forcing_sigma0(double amp, double alpha, double beta) {
     return amp * std::sqrt((1.0 - alpha * alpha) / (8.0 * beta * beta * s));
 }
 
+// planes per slab of the FP64 step's passes: slabs of equal thickness whose scratch stays within 1 GB (at
+// least 4 planes each).  A slab repeats the primitives of four planes and the predictors of two, so
+// thick ones: 256^3 8.60 ms within 1 GB, 8.94 ms within 256 MB, 10.7 ms within 64 MB, which L2 would hold.
+constexpr size_t PASS_SCRATCH_BYTES = (size_t)1 << 30;
+int pass_slab(int nx, int ny, int nz) {
+    int slabs = 1;
+    while ((nz + slabs - 1) / slabs > 4 && passes_scratch_bytes(nx, ny, (nz + slabs - 1) / slabs) > PASS_SCRATCH_BYTES)
+        ++slabs;
+    return (nz + slabs - 1) / slabs;
+}
+
 // Streams that the boxes of an ensemble fork over, one box each where there are enough.  A box's kernel
 // fills the chip for a part of its time only; with all boxes queued, blocks of others take the SMs it
 // leaves idle (64 uneven boxes, 41 M zones: 4.22 ms a step over 8 streams, 3.83 over 32, 3.65 over 64).
 // The single-box kernels run here, with a box's arguments in constant memory: a persistent kernel over
 // a queue of tiles of all boxes held them in registers, spilled, and took 3.95 ms.
-constexpr int ENS_LANES = 64;
+// In FP64 every lane has the passes' scratch of the largest box.
+constexpr int ENS_LANES = 64, ENS_LANES_F64 = 4;
 // Mean box below which two steps are replayed as a graph: a box's three launches take the host 7 us, about
 // what a 48^3 box takes the chip (64 boxes); above that plain launches keep the boxes' order, which the
 // graph's branches do not (41 M zones: 3.65 ms a step against 3.75 to 3.93).
@@ -126,6 +138,13 @@ struct gmt_ctx {
     struct CtTmaMap { const void* base; CUtensorMap map8, map1; };
     CtTmaMap ct_tma[2] = {};       // the same for the CT state (8 variables, and bzf alone)
     int ct_tma_next = 0;
+    // scratch of the FP64 step's passes (slabs of pass_S planes; null: the tile march).  Steps of one
+    // context on several streams or threads take it in turn: each waits for pass_ev, which the last
+    // one recorded behind its kernels.
+    void* pass = nullptr;
+    int pass_S = 0;
+    cudaEvent_t pass_ev = nullptr;
+    std::mutex pass_mu;
 };
 
 namespace {
@@ -318,6 +337,29 @@ template <class R> Planes<R> planes(void* base, size_t n) {
     return P;
 }
 
+// One unsplit step.  FP64 with automatic tiles runs as passes over the context's scratch; a call under
+// stream capture, which must not be ordered against work outside the captured graph, a context whose
+// tile the caller chose, and the failure-path tests keep the tile march.  Both give the same bits.
+template <class R> cudaError_t unsplit_step(gmt_ctx* c, const UnsplitArgs<R>& A, int riem, cudaStream_t s) {
+    if constexpr (std::is_same<R, double>::value) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (c->pass && !A.wait_test) {
+            if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+                cudaGetLastError();
+                cap = cudaStreamCaptureStatusActive;
+            }
+            if (cap == cudaStreamCaptureStatusNone) {
+                std::lock_guard<std::mutex> lk(c->pass_mu);
+                cudaError_t e = cudaStreamWaitEvent(s, c->pass_ev, 0);
+                if (e == cudaSuccess) e = launch_passes(A, c->p.recon, riem, c->pass, c->pass_S, s);
+                const cudaError_t e2 = cudaEventRecord(c->pass_ev, s);
+                return e != cudaSuccess ? e : e2;
+            }
+        }
+    }
+    return launch_unsplit(A, c->p.recon, riem, s);
+}
+
 template <class R>
 int step_impl(gmt_ctx* c, const CPlanes<R>& u, const Planes<R>& o, const gmt_step_args* a, cudaStream_t s,
               const void* const* sp_in = nullptr, void* const* sp_out = nullptr) {
@@ -351,7 +393,7 @@ int step_impl(gmt_ctx* c, const CPlanes<R>& u, const Planes<R>& o, const gmt_ste
             A.cfl_out = c->cfl;
         }
         int riem = p.riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : p.riemann;
-        cudaError_t e = launch_unsplit(A, p.recon, riem, s);
+        cudaError_t e = unsplit_step(c, A, riem, s);
         if (e != cudaSuccess) return cuda_fail(e, "unsplit step");
         return GMT_OK;
     }
@@ -557,6 +599,16 @@ int gmt_create(const gmt_params* p, gmt_ctx** out) {
     if (ok) ok = alloc((void**)&c->loop, sizeof(LoopState)) && alloc((void**)&c->loopc, sizeof(LoopConst)) &&
                  alloc(&c->bt, sizeof(BoxTables<double>));
     if (ok && cudaMemset(c->err, 0, sizeof(int)) != cudaSuccess) ok = false;
+    if (ok && p->scheme == GMT_SCHEME_UNSPLIT && c->esize == 8 && p->tile_x <= 0 && p->tile_y <= 0 && p->tile_z <= 0) {
+        // without the memory for it the tile march remains
+        c->pass_S = pass_slab(p->nx, p->ny, p->nz);
+        if (cudaMalloc(&c->pass, passes_scratch_bytes(p->nx, p->ny, c->pass_S)) != cudaSuccess ||
+            cudaEventCreateWithFlags(&c->pass_ev, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(c->pass);
+            c->pass = nullptr;
+        }
+    }
     if (!ok) { gmt_destroy(c); return GMT_ERR_NOMEM; }
     for (int a = 0; a < 3; ++a) {
         std::vector<double> t = trig_table(dims[a]);
@@ -621,6 +673,8 @@ int gmt_destroy(gmt_ctx* c) {
     cudaFree(c->spec);
     cudaFree(c->adj);
     cudaFree(c->adj_damp);
+    cudaFree(c->pass);
+    if (c->pass_ev) cudaEventDestroy(c->pass_ev);
     if (c->cap) cudaStreamDestroy(c->cap);
     cudaFree(c->loop);
     cudaFree(c->loopc);
@@ -1090,6 +1144,8 @@ cudaError_t run_enqueue(gmt_ctx* c, const void* src, void* dst, int flags, cudaS
     A.fmass = nullptr;
     set_tma(c, A);
     int riem = p.riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : p.riemann;
+    if constexpr (std::is_same<R, double>::value)   // gmt_run orders the whole run against pass_ev
+        if (c->pass && !A.wait_test) return launch_passes(A, p.recon, riem, c->pass, c->pass_S, s);
     return launch_unsplit(A, p.recon, riem, s);
 }
 
@@ -1116,6 +1172,11 @@ int gmt_run(gmt_ctx* c, void* u, void* w, int32_t nsteps, double t0, double t_en
     int rc = gmt_cfl_async(c, u, stream);   // CFL of the initial state; later steps fuse it
     if (rc) return rc;
     const int pairs = nsteps / 2;
+    std::unique_lock<std::mutex> turn(c->pass_mu, std::defer_lock);   // the passes' scratch, for the whole run
+    if (c->pass) {
+        turn.lock();
+        GMT_CUDA(cudaStreamWaitEvent(s, c->pass_ev, 0));
+    }
     if ((flags & GMT_RUN_GRAPH) && pairs > 0) {
         cudaGraphExec_t exec = nullptr;
         for (auto& g : c->graphs)
@@ -1147,6 +1208,7 @@ int gmt_run(gmt_ctx* c, void* u, void* w, int32_t nsteps, double t0, double t_en
         }
     }
     if (nsteps & 1) GMT_CUDA(run_enqueue_any(c, u, w, flags, s));
+    if (c->pass) GMT_CUDA(cudaEventRecord(c->pass_ev, s));
     int herr = 0;
     GMT_CUDA(cudaMemcpyAsync(&S, c->loop, sizeof(S), cudaMemcpyDeviceToHost, s));
     GMT_CUDA(cudaMemcpyAsync(&herr, c->err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1189,6 +1251,8 @@ struct gmt_ensemble {
     std::vector<cudaStream_t> lane;
     std::vector<cudaEvent_t> lane_ev;
     cudaEvent_t fork = nullptr;
+    std::vector<void*> pass;         // FP64: per lane, scratch of the step's passes
+    std::vector<int> pass_S;         // FP64: per box, planes of a slab
     int* err = nullptr;
     const int* mode_k_dev = nullptr;
     cudaStream_t cap = nullptr;
@@ -1270,6 +1334,14 @@ template <class R> void ens_bind(gmt_ensemble* E, void* const* u, void* const* w
         }
 }
 
+cudaError_t ens_launch(gmt_ensemble* E, const UnsplitArgs<float>& A, int, int, int riem, cudaStream_t s) {
+    return launch_unsplit(A, E->p.recon, riem, s);
+}
+cudaError_t ens_launch(gmt_ensemble* E, const UnsplitArgs<double>& A, int box, int lane, int riem, cudaStream_t s) {
+    if (E->pass[lane]) return launch_passes(A, E->p.recon, riem, E->pass[lane], E->pass_S[box], s);
+    return launch_unsplit(A, E->p.recon, riem, s);
+}
+
 // f() puts the boxes' work on the lanes, which are forked from s and joined to it again
 template <class F> cudaError_t ens_fork(gmt_ensemble* E, cudaStream_t s, F f) {
     const int L = (int)E->lane.size();
@@ -1304,7 +1376,7 @@ template <class R> cudaError_t ens_enqueue(gmt_ensemble* E, int par, int flags, 
         if (flags & GMT_RUN_FORCING)
             btab_cond_kernel<R><<<std::min((E->n[b] * E->n[b] + BTAB_ROWS - 1) / BTAB_ROWS, 32), 4 * BTAB_ROWS, 0, s>>>(
                 (const BoxTables<R>*)E->bt + b, E->loop + b, E->mode_k_dev);
-        e = launch_unsplit(A[par * E->nbox + b], E->p.recon, riem, s);
+        e = ens_launch(E, A[par * E->nbox + b], b, j % L, riem, s);
     }
     return e;
 }
@@ -1326,6 +1398,7 @@ int gmt_ensemble_destroy(gmt_ensemble* E) {
     for (cudaEvent_t v : E->lane_ev)
         if (v) cudaEventDestroy(v);
     if (E->fork) cudaEventDestroy(E->fork);
+    for (void* x : E->pass) cudaFree(x);
     for (void* x : E->trig8) cudaFree(x);
     cudaFree(E->loop);
     cudaFree(E->loopc);
@@ -1387,7 +1460,7 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
     }
 
     ens_tiles(E);
-    const int lanes = std::min(nbox, ENS_LANES);
+    const int lanes = std::min(nbox, E->esize == 8 ? ENS_LANES_F64 : ENS_LANES);
     E->lane.assign(lanes, nullptr);
     E->lane_ev.assign(lanes, nullptr);
     for (int i = 0; i < lanes; ++i) {
@@ -1395,6 +1468,19 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&E->lane_ev[i], cudaEventDisableTiming);
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&E->fork, cudaEventDisableTiming);
+    if (e == cudaSuccess && E->esize == 8) {
+        size_t need = 0;
+        for (int b = 0; b < nbox; ++b) {
+            E->pass_S.push_back(pass_slab(n[b], n[b], n[b]));
+            need = std::max(need, passes_scratch_bytes(n[b], n[b], E->pass_S[b]));
+        }
+        E->pass.assign(lanes, nullptr);
+        for (void*& x : E->pass)
+            if (cudaMalloc(&x, need) != cudaSuccess) {   // that lane keeps the tile march
+                cudaGetLastError();
+                x = nullptr;
+            }
+    }
     if (e == cudaSuccess) e = cudaMemset(E->err, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(E->modes, 0, (size_t)nbox * NMODES * 6 * sizeof(double));
     if (e == cudaSuccess) e = mode_table_device(&E->mode_k_dev);

@@ -14,6 +14,9 @@ constexpr int NMODES = 61;
 // unsplit GLM step (gmt_unsplit_f32.cu / gmt_unsplit_f64.cu)
 cudaError_t launch_unsplit(const UnsplitArgs<float>& A, int recon, int riem, cudaStream_t s);
 cudaError_t launch_unsplit(const UnsplitArgs<double>& A, int recon, int riem, cudaStream_t s);
+// the FP64 step as three passes over z slabs of S planes with caller-supplied scratch
+cudaError_t launch_passes(const UnsplitArgs<double>& A, int recon, int riem, void* scratch, int S, cudaStream_t s);
+size_t passes_scratch_bytes(int nx, int ny, int S);
 int unsplit_max_threads(int dtype_bytes);
 cudaError_t unsplit_prepare_f32();   // shared-memory attributes of every step kernel
 cudaError_t unsplit_prepare_f64();

@@ -1,5 +1,8 @@
 // FP64 unsplit step kernels: up to 256 threads, 1 resident block per SM.  Built with --fmad=false
 // so each expression rounds exactly as the IEEE evaluation of the oracle.
+#include <algorithm>
+
+#include "gmt_passes.cuh"
 #include "gmt_unsplit_inst.cuh"
 
 namespace gmt {
@@ -18,6 +21,43 @@ cudaError_t launch_unsplit(const UnsplitArgs<double>& A, int recon, int riem, cu
     cudaError_t e = cudaSuccess;
     if (fixed_tile64<32, 8>(A, recon, riem, s, e) || fixed_tile64<16, 16>(A, recon, riem, s, e)) return e;
     return unsplit_dispatch_t<double, 256, 1>(A, recon, riem, s);
+}
+// The step as three passes over z slabs of S planes (gmt_passes.cuh); scratch of passes_scratch_bytes.
+size_t passes_scratch_bytes(int nx, int ny, int S) {
+    return (size_t)nx * ny * ((size_t)9 * (2 * S + 6) * sizeof(double) + (S + 2));
+}
+constexpr int PTX = 16, PTY = 8, PMINB = 4;
+template <int RECON, int RIEM>
+static cudaError_t passes_go(const UnsplitArgs<double>& A, void* scratch, int S, cudaStream_t s) {
+    const size_t nxy = (size_t)A.nx * A.ny;
+    PassArgs<double> P;
+    P.A = A;
+    const int bx = (A.nx + PTX - 1) / PTX, by = (A.ny + PTY - 1) / PTY;
+    for (P.zs = 0; P.zs < A.nz; P.zs += S) {
+        P.S = std::min(S, A.nz - P.zs);
+        P.q = static_cast<double*>(scratch);
+        P.mh = P.q + 9 * nxy * (P.S + 4);
+        P.up = reinterpret_cast<unsigned char*>(P.mh + 9 * nxy * (P.S + 2));
+        pass_prim_kernel<double><<<dim3((unsigned)((nxy + 255) / 256), P.S + 4), 256, 0, s>>>(P);
+        pass_recon_kernel<double, RECON><<<dim3((unsigned)((nxy + 127) / 128), P.S + 2), 128, 0, s>>>(P);
+        // planes per block of the flux pass: the extra z face of a chunk costs a third of a plane, so
+        // long chunks, but enough blocks for several rounds of PMINB blocks on every SM
+        int lz = P.S;
+        while (lz > 4 && (long)bx * by * ((P.S + lz - 1) / lz) < 148L * PMINB * 3) lz = (lz + 1) / 2;
+        P.lz = lz;
+        pass_flux_kernel<double, RECON, RIEM, PTX, PTY, PMINB>
+            <<<dim3(bx, by, (P.S + lz - 1) / lz), PTX * PTY, pass_flux_smem<PTX, PTY>(sizeof(double)), s>>>(P);
+    }
+    return cudaGetLastError();
+}
+cudaError_t launch_passes(const UnsplitArgs<double>& A, int recon, int riem, void* scratch, int S, cudaStream_t s) {
+#define GMT_CASE(RC, RM) \
+    if (recon == RC && riem == RM) return passes_go<RC, RM>(A, scratch, S, s);
+    GMT_CASE(RECON_MC, RIEM_HLLD) GMT_CASE(RECON_MC, RIEM_HLL) GMT_CASE(RECON_MC, RIEM_LLF_BOUND)
+    GMT_CASE(RECON_MINMOD, RIEM_HLLD) GMT_CASE(RECON_MINMOD, RIEM_HLL) GMT_CASE(RECON_MINMOD, RIEM_LLF_BOUND)
+    GMT_CASE(RECON_PPM, RIEM_HLLD) GMT_CASE(RECON_PPM, RIEM_HLL) GMT_CASE(RECON_PPM, RIEM_LLF_BOUND)
+#undef GMT_CASE
+    return cudaErrorInvalidValue;
 }
 cudaError_t unsplit_prepare_f64() {
     cudaError_t e = unsplit_configure_all_t<double, 256, 1>();
