@@ -171,12 +171,16 @@ template <class R> Consts<R> consts_of(const gmt_params& p) {
 int choose_chunk(long cols, int nz) {
     // a block takes lz planes and 2.8 planes' time for its start and for the first and last planes, which
     // only reconstruct (64^3, chunk 4 -> 64: 41 -> 401 us, 6.05 us a plane)
+    // Four planes at least.  Shorter chunks finish a small box that has the chip to itself sooner (32^3:
+    // 20 us at 1, 33 at 3, 39 at 4; 48^3: 29 at 2, 41 at 4; with one chunk a tile 64 and 46), but more than
+    // 40 % of each block is then its start.  Looping over single boxes is to stay at no more than half of the
+    // ensemble's rate, which the loop's small boxes at 1 or 2 planes broke (5.65 against 11.2 Gzone/s; now 5.26).
     constexpr double start = 2.8;
     double best = 1e300;
     int last = 0, choice = nz;
     for (int nch = 1; nch <= std::min(nz, 4096); ++nch) {
         const int lz = (nz + nch - 1) / nch;
-        if (lz == last) continue;
+        if (lz == last || (lz < 4 && nch > 1)) continue;
         last = lz;
         const long rounds = (cols * ((nz + lz - 1) / lz) + 147) / 148;
         const double cost = ((double)rounds + (rounds > 1 ? 0.2 : 0.0)) * (lz + start);
