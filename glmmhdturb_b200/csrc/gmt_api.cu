@@ -69,17 +69,6 @@ double forcing_sigma0(double amp, double alpha, double beta) {
     return amp * std::sqrt((1.0 - alpha * alpha) / (8.0 * beta * beta * s));
 }
 
-// planes per slab of the FP64 step's passes: slabs of equal thickness whose scratch stays within 1 GB (at
-// least 4 planes each).  A slab repeats the primitives of four planes and the predictors of two, so
-// thick ones: 256^3 8.60 ms within 1 GB, 8.94 ms within 256 MB, 10.7 ms within 64 MB, which L2 would hold.
-constexpr size_t PASS_SCRATCH_BYTES = (size_t)1 << 30;
-int pass_slab(int nx, int ny, int nz) {
-    int slabs = 1;
-    while ((nz + slabs - 1) / slabs > 4 && passes_scratch_bytes(nx, ny, (nz + slabs - 1) / slabs) > PASS_SCRATCH_BYTES)
-        ++slabs;
-    return (nz + slabs - 1) / slabs;
-}
-
 // Streams that the boxes of an ensemble fork over, one box each where there are enough.  A box's kernel
 // fills the chip for a part of its time only; with all boxes queued, blocks of others take the SMs it
 // leaves idle (64 uneven boxes, 41 M zones: 4.22 ms a step over 8 streams, 3.83 over 32, 3.65 over 64).
@@ -604,10 +593,11 @@ int gmt_create(const gmt_params* p, gmt_ctx** out) {
                  alloc(&c->bt, sizeof(BoxTables<double>));
     if (ok && cudaMemset(c->err, 0, sizeof(int)) != cudaSuccess) ok = false;
     if (ok && p->scheme == GMT_SCHEME_UNSPLIT && c->esize == 8 && p->tile_x <= 0 && p->tile_y <= 0 && p->tile_z <= 0) {
-        // without the memory for it the tile march remains
+        // without slabs or the memory for them the tile march remains
         c->pass_S = pass_slab(p->nx, p->ny, p->nz);
-        if (cudaMalloc(&c->pass, passes_scratch_bytes(p->nx, p->ny, c->pass_S)) != cudaSuccess ||
-            cudaEventCreateWithFlags(&c->pass_ev, cudaEventDisableTiming) != cudaSuccess) {
+        if (c->pass_S > 0 &&
+            (cudaMalloc(&c->pass, passes_scratch_bytes(p->nx, p->ny, c->pass_S)) != cudaSuccess ||
+             cudaEventCreateWithFlags(&c->pass_ev, cudaEventDisableTiming) != cudaSuccess)) {
             cudaGetLastError();
             cudaFree(c->pass);
             c->pass = nullptr;
@@ -1342,7 +1332,7 @@ cudaError_t ens_launch(gmt_ensemble* E, const UnsplitArgs<float>& A, int, int, i
     return launch_unsplit(A, E->p.recon, riem, s);
 }
 cudaError_t ens_launch(gmt_ensemble* E, const UnsplitArgs<double>& A, int box, int lane, int riem, cudaStream_t s) {
-    if (E->pass[lane]) return launch_passes(A, E->p.recon, riem, E->pass[lane], E->pass_S[box], s);
+    if (E->pass[lane] && E->pass_S[box] > 0) return launch_passes(A, E->p.recon, riem, E->pass[lane], E->pass_S[box], s);
     return launch_unsplit(A, E->p.recon, riem, s);
 }
 
@@ -1476,11 +1466,11 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
         size_t need = 0;
         for (int b = 0; b < nbox; ++b) {
             E->pass_S.push_back(pass_slab(n[b], n[b], n[b]));
-            need = std::max(need, passes_scratch_bytes(n[b], n[b], E->pass_S[b]));
+            if (E->pass_S[b] > 0) need = std::max(need, passes_scratch_bytes(n[b], n[b], E->pass_S[b]));
         }
         E->pass.assign(lanes, nullptr);
         for (void*& x : E->pass)
-            if (cudaMalloc(&x, need) != cudaSuccess) {   // that lane keeps the tile march
+            if (need > 0 && cudaMalloc(&x, need) != cudaSuccess) {   // that lane keeps the tile march
                 cudaGetLastError();
                 x = nullptr;
             }

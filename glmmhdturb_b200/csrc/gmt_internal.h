@@ -6,6 +6,7 @@
 #include <string>
 
 #include "gmt_common.cuh"
+#include "gmt_plan.h"
 
 namespace gmt {
 
@@ -16,7 +17,6 @@ cudaError_t launch_unsplit(const UnsplitArgs<float>& A, int recon, int riem, cud
 cudaError_t launch_unsplit(const UnsplitArgs<double>& A, int recon, int riem, cudaStream_t s);
 // the FP64 step as three passes over z slabs of S planes with caller-supplied scratch
 cudaError_t launch_passes(const UnsplitArgs<double>& A, int recon, int riem, void* scratch, int S, cudaStream_t s);
-size_t passes_scratch_bytes(int nx, int ny, int S);
 int unsplit_max_threads(int dtype_bytes);
 cudaError_t unsplit_prepare_f32();   // shared-memory attributes of every step kernel
 cudaError_t unsplit_prepare_f64();

@@ -23,10 +23,7 @@ cudaError_t launch_unsplit(const UnsplitArgs<double>& A, int recon, int riem, cu
     return unsplit_dispatch_t<double, 256, 1>(A, recon, riem, s);
 }
 // The step as three passes over z slabs of S planes (gmt_passes.cuh); scratch of passes_scratch_bytes.
-size_t passes_scratch_bytes(int nx, int ny, int S) {
-    return (size_t)nx * ny * ((size_t)9 * (2 * S + 6) * sizeof(double) + (S + 2));
-}
-constexpr int PTX = 16, PTY = 8, PMINB = 4;
+constexpr int PTX = PASS_TX, PTY = PASS_TY, PMINB = 4;
 template <int RECON, int RIEM>
 static cudaError_t passes_go(const UnsplitArgs<double>& A, void* scratch, int S, cudaStream_t s) {
     const size_t nxy = (size_t)A.nx * A.ny;
@@ -40,6 +37,8 @@ static cudaError_t passes_go(const UnsplitArgs<double>& A, void* scratch, int S,
         P.up = reinterpret_cast<unsigned char*>(P.mh + 9 * nxy * (P.S + 2));
         pass_prim_kernel<double><<<dim3((unsigned)((nxy + 255) / 256), P.S + 4), 256, 0, s>>>(P);
         pass_recon_kernel<double, RECON><<<dim3((unsigned)((nxy + 127) / 128), P.S + 2), 128, 0, s>>>(P);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;   // no fluxes from scratch that was not written
         // planes per block of the flux pass: the extra z face of a chunk costs a third of a plane, so
         // long chunks, but enough blocks for several rounds of PMINB blocks on every SM
         int lz = P.S;

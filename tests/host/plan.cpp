@@ -1,0 +1,21 @@
+// Prints what the rules of gmt_plan.h choose.  One query per line of standard input, one answer per line:
+//   slab nx ny nz     -> planes per slab of the FP64 passes, bytes of their scratch
+#include <cstdio>
+#include <cstring>
+
+#include "../../glmmhdturb_b200/csrc/gmt_plan.h"
+
+int main() {
+    char what[32];
+    while (std::scanf("%31s", what) == 1) {
+        if (!std::strcmp(what, "slab")) {
+            int nx, ny, nz;
+            if (std::scanf("%d %d %d", &nx, &ny, &nz) != 3) return 1;
+            const int S = gmt::pass_slab(nx, ny, nz);
+            std::printf("%d %zu\n", S, gmt::passes_scratch_bytes(nx, ny, S));
+        } else {
+            return 1;
+        }
+    }
+    return 0;
+}

@@ -44,6 +44,20 @@ def test_slabs():
     assert torch.equal(x, y)
 
 
+def test_more_planes_than_a_launch_takes():
+    """A narrow box whose planes exceed gridDim.y (65535) in one slab, though their scratch would fit one."""
+    from glmmhdturb_b200 import Solver
+    n = (8, 4, 70000)
+    a, b = Solver(n, dtype="f64", gamma=5 / 3), Solver(n, dtype="f64", gamma=5 / 3, tile=(8, 4, 0))
+    u = a.alloc()
+    a.ic_turbulent(u, mach=1.0, seed=3)
+    x, y = torch.full_like(u, float("nan")), torch.empty_like(u)
+    for s, o in ((a, x), (b, y)):
+        s.step(u, o, 0.02 * s.dx, ch=3.0, glm_fac=0.99, want_cfl=True)
+    assert torch.equal(x, y)
+    assert a.cfl_result() == b.cfl_result()
+
+
 def test_under_capture_and_after():
     """A captured step takes the tile march (it must not be ordered against work outside its graph)."""
     from glmmhdturb_b200 import Solver
