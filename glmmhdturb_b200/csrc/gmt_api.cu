@@ -74,7 +74,7 @@ double forcing_sigma0(double amp, double alpha, double beta) {
 // leaves idle (64 uneven boxes, 41 M zones: 4.22 ms a step over 8 streams, 3.83 over 32, 3.65 over 64).
 // The single-box kernels run here, with a box's arguments in constant memory: a persistent kernel over
 // a queue of tiles of all boxes held them in registers, spilled, and took 3.95 ms.
-// In FP64 every lane has the passes' scratch of the largest box.
+// In FP64 every lane has the passes' scratch of the largest box, an equal share of a context's at most.
 constexpr int ENS_LANES = 64, ENS_LANES_F64 = 4;
 // Mean box below which two steps are replayed as a graph: a box's three launches take the host 7 us, about
 // what a 48^3 box takes the chip (64 boxes); above that plain launches keep the boxes' order, which the
@@ -594,7 +594,7 @@ int gmt_create(const gmt_params* p, gmt_ctx** out) {
     if (ok && cudaMemset(c->err, 0, sizeof(int)) != cudaSuccess) ok = false;
     if (ok && p->scheme == GMT_SCHEME_UNSPLIT && c->esize == 8 && p->tile_x <= 0 && p->tile_y <= 0 && p->tile_z <= 0) {
         // without slabs or the memory for them the tile march remains
-        c->pass_S = pass_slab(p->nx, p->ny, p->nz);
+        c->pass_S = pass_slab(p->nx, p->ny, p->nz, PASS_SCRATCH_BYTES);
         if (c->pass_S > 0 &&
             (cudaMalloc(&c->pass, passes_scratch_bytes(p->nx, p->ny, c->pass_S)) != cudaSuccess ||
              cudaEventCreateWithFlags(&c->pass_ev, cudaEventDisableTiming) != cudaSuccess)) {
@@ -1465,7 +1465,7 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
     if (e == cudaSuccess && E->esize == 8) {
         size_t need = 0;
         for (int b = 0; b < nbox; ++b) {
-            E->pass_S.push_back(pass_slab(n[b], n[b], n[b]));
+            E->pass_S.push_back(pass_slab(n[b], n[b], n[b], PASS_SCRATCH_BYTES / lanes));
             if (E->pass_S[b] > 0) need = std::max(need, passes_scratch_bytes(n[b], n[b], E->pass_S[b]));
         }
         E->pass.assign(lanes, nullptr);

@@ -98,7 +98,9 @@ const char* gmt_version(void);
 const char* gmt_last_error(void);
 /* fill reference defaults for an n^3 box (glmmhd_turb.jl:28-52) */
 int gmt_params_init(gmt_params* p, int n);
-/* allocate a context on the current device: scratch for reductions, forcing tables, tiles */
+/* allocate a context on the current device: scratch for reductions, forcing tables, tiles; for the FP64
+ * unsplit step with automatic tiles also the scratch of its passes, at most 1 GB (without that memory, or
+ * where a cross section needs more, the step runs as the tile march, with the same bits) */
 int gmt_create(const gmt_params* p, gmt_ctx** out);
 int gmt_destroy(gmt_ctx* ctx);
 /* kernel resource report: registers, dynamic shared bytes and tile of the step kernel */
@@ -140,7 +142,8 @@ int gmt_run(gmt_ctx* ctx, void* u, void* w, int32_t nsteps, double t0, double t_
  * (no counterpart in the reference).  Every box: its own n^3 grid (n a multiple of 16), forcing
  * amplitude and seed; the physics of `base`.  Each box advances on a stream of its own, forked from
  * the caller's: a tick, the conditional forcing update and its step kernel per step, ordered only
- * after the box's own previous step, so the boxes fill the chip together. */
+ * after the box's own previous step, so the boxes fill the chip together.  An FP64 ensemble takes up to
+ * 1 GB of scratch for its steps. */
 typedef struct gmt_ensemble gmt_ensemble;
 int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, const double* turb_amp,
                         const uint32_t* seeds, gmt_ensemble** out);

@@ -1,5 +1,5 @@
 // Prints what the rules of gmt_plan.h choose.  One query per line of standard input, one answer per line:
-//   slab nx ny nz     -> planes per slab of the FP64 passes, bytes of their scratch
+//   slab nx ny nz lanes -> planes per slab of the FP64 passes of one of `lanes` lanes, bytes of their scratch
 #include <cstdio>
 #include <cstring>
 
@@ -9,10 +9,10 @@ int main() {
     char what[32];
     while (std::scanf("%31s", what) == 1) {
         if (!std::strcmp(what, "slab")) {
-            int nx, ny, nz;
-            if (std::scanf("%d %d %d", &nx, &ny, &nz) != 3) return 1;
-            const int S = gmt::pass_slab(nx, ny, nz);
-            std::printf("%d %zu\n", S, gmt::passes_scratch_bytes(nx, ny, S));
+            int nx, ny, nz, lanes;
+            if (std::scanf("%d %d %d %d", &nx, &ny, &nz, &lanes) != 4) return 1;
+            const int S = gmt::pass_slab(nx, ny, nz, gmt::PASS_SCRATCH_BYTES / lanes);
+            std::printf("%d %zu\n", S, S > 0 ? gmt::passes_scratch_bytes(nx, ny, S) : (size_t)0);
         } else {
             return 1;
         }

@@ -29,13 +29,29 @@ def plan(tmp_path_factory):
 
 # narrow boxes of many planes and of many rows among ordinary ones, all within gmt_create's 4e9 cells
 @pytest.mark.parametrize("n", [(1, 1, 1), (16, 16, 16), (192, 192, 192), (512, 512, 512), (8, 8, 65531), (8, 8, 65532),
-                               (8, 8, 70000), (1, 1, 2000000000), (4, 524280, 2), (4, 524281, 2), (1, 2000000000, 1)])
+                               (8, 8, 70000), (1, 1, 2000000000), (1, 524280, 2), (1, 524281, 2), (1, 2000000000, 1)])
 def test_fp64_passes_fit_the_grid_limits(plan, n):
     """The primitive and predictor passes launch a slab's planes and four (two) more in gridDim.y, the flux
     pass the rows of its tiles; a box that this does not fit has no slab and takes the tile march."""
-    (S, _), = plan(("slab", *n))
+    (S, _), = plan(("slab", *n, 1))
     assert 0 <= S <= n[2]
     if -(-n[1] // PASS_TY) > GRID_YZ:
         assert S == 0
     else:
         assert 1 <= S and S + 4 <= GRID_YZ
+
+
+# cross sections around the one whose four planes just fit, thin and thick; the boxes of an ensemble
+@pytest.mark.parametrize("n", [(192, 192, 192), (1024, 1024, 3), (1024, 1024, 64), (1029, 1029, 64), (1030, 1030, 64),
+                               (1536, 1536, 3), (1536, 1536, 128), (2048, 2048, 256), (1024, 1024, 9), (512, 512, 512), (528, 528, 528)])
+@pytest.mark.parametrize("lanes", [1, 3, 4])
+def test_fp64_scratch_stays_within_its_budget(plan, n, lanes):
+    """The passes' scratch is at most 1 GB for a context and for all lanes of an ensemble together; slabs are cut
+    down to three or four planes (or the box's, if it has fewer), and a box that still exceeds it has none."""
+    (S, size), = plan(("slab", *n, lanes))
+    budget = (1 << 30) // lanes
+    if S == 0:   # 9 planes of primitives and of predictors in 8 bytes, 4 and 2 more than the slab; 1-byte flags
+        k = min(4, n[2])
+        assert n[0] * n[1] * (72 * (2 * k + 6) + k + 2) > budget
+    else:
+        assert S >= min(3, n[2]) and size <= budget
