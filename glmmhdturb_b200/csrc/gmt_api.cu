@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -11,6 +12,7 @@
 #include "gmt_internal.h"
 #include "gmt_unsplit.cuh"
 #include "gmt_loop.cuh"
+#include "gmt_turn.h"
 
 using namespace gmt;
 
@@ -128,8 +130,8 @@ struct gmt_ctx {
     CtTmaMap ct_tma[2] = {};       // the same for the CT state (8 variables, and bzf alone)
     int ct_tma_next = 0;
     // scratch of the FP64 step's passes (slabs of pass_S planes; null: the tile march).  Steps of one
-    // context on several streams or threads take it in turn: each waits for pass_ev, which the last
-    // one recorded behind its kernels.
+    // context on several streams or threads take it in turn (ScratchTurn).  It alone is shared so: the CFL
+    // words, the forcing and loop records and the tensor maps are the caller's to keep apart.
     void* pass = nullptr;
     int pass_S = 0;
     cudaEvent_t pass_ev = nullptr;
@@ -342,10 +344,10 @@ template <class R> cudaError_t unsplit_step(gmt_ctx* c, const UnsplitArgs<R>& A,
                 cap = cudaStreamCaptureStatusActive;
             }
             if (cap == cudaStreamCaptureStatusNone) {
-                std::lock_guard<std::mutex> lk(c->pass_mu);
-                cudaError_t e = cudaStreamWaitEvent(s, c->pass_ev, 0);
-                if (e == cudaSuccess) e = launch_passes(A, c->p.recon, riem, c->pass, c->pass_S, s);
-                const cudaError_t e2 = cudaEventRecord(c->pass_ev, s);
+                ScratchTurn turn(c->pass_mu, c->pass_ev, s);
+                if (turn.status() != cudaSuccess) return turn.status();
+                const cudaError_t e = launch_passes(A, c->p.recon, riem, c->pass, c->pass_S, s);
+                const cudaError_t e2 = turn.mark();
                 return e != cudaSuccess ? e : e2;
             }
         }
@@ -1166,10 +1168,10 @@ int gmt_run(gmt_ctx* c, void* u, void* w, int32_t nsteps, double t0, double t_en
     int rc = gmt_cfl_async(c, u, stream);   // CFL of the initial state; later steps fuse it
     if (rc) return rc;
     const int pairs = nsteps / 2;
-    std::unique_lock<std::mutex> turn(c->pass_mu, std::defer_lock);   // the passes' scratch, for the whole run
+    std::optional<ScratchTurn> turn;   // the passes' scratch, for the whole run
     if (c->pass) {
-        turn.lock();
-        GMT_CUDA(cudaStreamWaitEvent(s, c->pass_ev, 0));
+        turn.emplace(c->pass_mu, c->pass_ev, s);
+        GMT_CUDA(turn->status());
     }
     if ((flags & GMT_RUN_GRAPH) && pairs > 0) {
         cudaGraphExec_t exec = nullptr;
@@ -1202,7 +1204,7 @@ int gmt_run(gmt_ctx* c, void* u, void* w, int32_t nsteps, double t0, double t_en
         }
     }
     if (nsteps & 1) GMT_CUDA(run_enqueue_any(c, u, w, flags, s));
-    if (c->pass) GMT_CUDA(cudaEventRecord(c->pass_ev, s));
+    if (turn) GMT_CUDA(turn->mark());
     int herr = 0;
     GMT_CUDA(cudaMemcpyAsync(&S, c->loop, sizeof(S), cudaMemcpyDeviceToHost, s));
     GMT_CUDA(cudaMemcpyAsync(&herr, c->err, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -1,4 +1,5 @@
-"""The rules that cut a step up for its grid (gmt_plan.h), on the CPU: tests/host/plan.cpp prints their choices."""
+"""Host code of the library without a GPU: the rules that cut a step up for its grid (gmt_plan.h; tests/host/plan.cpp
+prints their choices), and the turns at shared scratch (gmt_turn.h)."""
 import os
 import shutil
 import subprocess
@@ -55,3 +56,23 @@ def test_fp64_scratch_stays_within_its_budget(plan, n, lanes):
         assert n[0] * n[1] * (72 * (2 * k + 6) + k + 2) > budget
     else:
         assert S >= min(3, n[2]) and size <= budget
+
+
+def test_scratch_is_handed_on_however_a_holder_leaves(tmp_path):
+    """ScratchTurn (gmt_turn.h) over stand-ins of the runtime calls (tests/host/turn.cpp): a holder that leaves
+    by an error exit after launching has its work marked like any other; one that could not wait for the last
+    holder neither launches nor marks; work that cannot be marked is waited for."""
+    cuda = "/usr/local/cuda/include"
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx or not os.path.exists(os.path.join(cuda, "cuda_runtime_api.h")):
+        pytest.skip("no C++ compiler or CUDA headers")
+    exe = str(tmp_path / "turn")
+    subprocess.run([cxx, "-std=c++17", "-O1", "-Wall", "-Werror", "-pthread", "-I", cuda, "-o", exe,
+                    os.path.join(HERE, "host", "turn.cpp")], check=True)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True, timeout=60).stdout
+    got = [s.split("\n")[:-1] for s in out.split("end\n")[:-1]]
+    assert got[0] == ["wait 1", "launch 1", "record 1", "status 0", "free 1"]
+    assert got[1] == ["wait 1", "launch 1", "record 1", "status 1", "free 1"]
+    assert got[2] == ["wait 1", "status 1", "free 1"]
+    assert got[3] == ["wait 1", "launch 1", "record 1", "synchronise 1", "status 1", "free 1"]
+    assert got[4] == ["wait 1", "launch 1", "record 1", "wait 2", "launch 2", "record 2"]
