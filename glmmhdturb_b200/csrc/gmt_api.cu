@@ -153,33 +153,6 @@ template <class R> Consts<R> consts_of(const gmt_params& p) {
     return K;
 }
 
-// The z chunk that fills the chip best: the number of rounds of blocks over the 148 SMs times the
-// length of a block.  Short chunks repeat the fixed part, long ones leave SMs idle in the last round;
-// with more than one round a share of a block's time is added, because blocks do not end together.
-// (FP32 MC + HLLD, chunk -> us: 64^3 4 -> 41, 8 -> 66; 96^3 12 -> 92, 6 -> 105; 192^3 32 -> 694,
-// 6 -> 833; 256^3 32 -> 1549, 16 -> 1623; 512^3 128 -> 11.59 ms, 64 and 256 -> 11.70 ms; the second
-// figures of the first four are the chunks of a rule that only asked for eight rounds of blocks.)
-int choose_chunk(long cols, int nz) {
-    // a block takes lz planes and 2.8 planes' time for its start and for the first and last planes, which
-    // only reconstruct (64^3, chunk 4 -> 64: 41 -> 401 us, 6.05 us a plane)
-    // Four planes at least.  Shorter chunks finish a small box that has the chip to itself sooner (32^3:
-    // 20 us at 1, 33 at 3, 39 at 4; 48^3: 29 at 2, 41 at 4; with one chunk a tile 64 and 46), but more than
-    // 40 % of each block is then its start.  Looping over single boxes is to stay at no more than half of the
-    // ensemble's rate, which the loop's small boxes at 1 or 2 planes broke (5.65 against 11.2 Gzone/s; now 5.26).
-    constexpr double start = 2.8;
-    double best = 1e300;
-    int last = 0, choice = nz;
-    for (int nch = 1; nch <= std::min(nz, 4096); ++nch) {
-        const int lz = (nz + nch - 1) / nch;
-        if (lz == last || (lz < 4 && nch > 1)) continue;
-        last = lz;
-        const long rounds = (cols * ((nz + lz - 1) / lz) + 147) / 148;
-        const double cost = ((double)rounds + (rounds > 1 ? 0.2 : 0.0)) * (lz + start);
-        if (cost < best) { best = cost; choice = lz; }
-    }
-    return choice;
-}
-
 int choose_tile(gmt_ctx* c, bool ct = false) {
     const gmt_params& p = c->p;
     const int maxt = ct ? ct_max_threads(c->esize) : unsplit_max_threads(c->esize);
@@ -202,7 +175,7 @@ int choose_tile(gmt_ctx* c, bool ct = false) {
         if (ox * oy > maxt) return fail(GMT_ERR_ARG, "tile_x*tile_y must be <= " + std::to_string(maxt));
         if (smem(ox, oy) > 227 * 1024) return fail(GMT_ERR_ARG, "tile needs more than 227 KB shared memory");
     }
-    const int lz = p.tile_z > 0 ? p.tile_z : choose_chunk(cols(ox, oy), p.nz);
+    const int lz = p.tile_z > 0 ? p.tile_z : choose_chunk(cols(ox, oy), p.nz, c->esize, ox * oy);
     c->ox = ox; c->oy = oy; c->lz = std::min(lz, p.nz);
     return GMT_OK;
 }

@@ -31,4 +31,46 @@ inline int pass_slab(int nx, int ny, int nz, size_t budget) {
     return over() ? 0 : planes();
 }
 
+// --- z chunks of the tile marches ----------------------------------------------------------------
+// Planes per block of `threads` columns in reals of `esize` bytes, `cols` tiles wide: the z chunk that fills the
+// chip best.
+//
+// A tile whose block fills an SM (FP32 above 256 threads, of 128 registers; FP64 from 128 threads, by its
+// shared memory; the automatic tiles are all of this kind): the number of rounds of blocks over the 148 SMs
+// times the length of a block.  Short chunks repeat the fixed part, long ones leave SMs idle in the last round;
+// with more than one round a share of a block's time is added, because blocks do not end together.
+// (FP32 MC + HLLD, chunk -> us: 64^3 4 -> 41, 8 -> 66; 96^3 12 -> 92, 6 -> 105; 192^3 32 -> 694,
+// 6 -> 833; 256^3 32 -> 1549, 16 -> 1623; 512^3 128 -> 11.59 ms, 64 and 256 -> 11.70 ms; the second
+// figures of the first four are the chunks of a rule that only asked for eight rounds of blocks.)
+//
+// Of smaller tiles, which a caller may choose, several blocks share an SM and hide one another's start, and
+// one block for each SM leaves most of it idle: halved until there are eight rounds of blocks, or 8 planes.
+// (FP32 MC + HLLD, us, that rule -> one block for each SM: 16x8 at 128^3 342 -> 729, 8x8 at 64^3 76 -> 204,
+// 32x4 at 128^3 368 -> 747, 16x16 at 256^3 1454 -> 1531; FP64 8x8 at 128x64x96 975 -> 2792.)
+inline int choose_chunk(long cols, int nz, int esize, int threads) {
+    if (esize == 8 ? threads < 128 : threads <= 256) {
+        long lz = nz;
+        while (lz > 8 && cols * ((nz + lz - 1) / lz) < 148L * 8) lz = (lz + 1) / 2;
+        return (int)lz;
+    }
+    // a block takes lz planes and 2.8 planes' time for its start and for the first and last planes, which
+    // only reconstruct (64^3, chunk 4 -> 64: 41 -> 401 us, 6.05 us a plane)
+    // Four planes at least.  Shorter chunks finish a small box that has the chip to itself sooner (32^3:
+    // 20 us at 1, 33 at 3, 39 at 4; 48^3: 29 at 2, 41 at 4; with one chunk a tile 64 and 46), but more than
+    // 40 % of each block is then its start.  Looping over single boxes is to stay at no more than half of the
+    // ensemble's rate, which the loop's small boxes at 1 or 2 planes broke (5.65 against 11.2 Gzone/s; now 5.26).
+    constexpr double start = 2.8;
+    double best = 1e300;
+    int last = 0, choice = nz;
+    for (int nch = 1; nch <= std::min(nz, 4096); ++nch) {
+        const int lz = (nz + nch - 1) / nch;
+        if (lz == last || (lz < 4 && nch > 1)) continue;
+        last = lz;
+        const long rounds = (cols * (((long)nz + lz - 1) / lz) + 147) / 148;
+        const double cost = ((double)rounds + (rounds > 1 ? 0.2 : 0.0)) * (lz + start);
+        if (cost < best) { best = cost; choice = lz; }
+    }
+    return choice;
+}
+
 }  // namespace gmt

@@ -58,6 +58,34 @@ def test_fp64_scratch_stays_within_its_budget(plan, n, lanes):
         assert S >= min(3, n[2]) and size <= budget
 
 
+# us a step of a tile march: with the rule that asked for eight rounds of blocks and no more (the kernels of
+# that time), and by planes per block.  Tiles of which several blocks share an SM:
+CHUNK_TIMES = [
+    ("unsplit mc", (64, 64, 64), "f32", (8, 8), 82, {4: 86, 6: 71, 8: 76, 12: 97, 16: 114, 24: 163, 32: 204, 64: 351}),
+    ("unsplit mc", (64, 64, 64), "f32", (16, 8), 67, {4: 77, 6: 59, 8: 62, 12: 87, 16: 106, 24: 137, 32: 178, 64: 329}),
+    ("unsplit ppm", (64, 64, 64), "f32", (32, 4), 104, {4: 131, 6: 95, 8: 104, 12: 142, 16: 175, 24: 243, 32: 315, 64: 603}),
+    ("unsplit mc", (128, 128, 128), "f32", (16, 8), 380, {4: 405, 6: 363, 8: 342, 12: 331, 16: 353, 24: 349, 32: 437, 64: 410, 128: 729}),
+    ("unsplit ppm", (128, 128, 128), "f32", (32, 8), 547, {4: 530, 6: 511, 8: 517, 12: 540, 16: 513, 24: 668, 32: 514, 64: 736, 128: 1419}),
+    ("unsplit mc", (128, 128, 128), "f32", (16, 16), 308, {4: 241, 6: 228, 8: 228, 12: 228, 16: 222, 24: 267, 32: 223, 64: 337, 128: 599}),
+    ("march1d mc", (128, 128, 128), "f32", (16, 8), 308, {4: 332, 6: 293, 8: 279, 12: 270, 16: 287, 24: 283, 32: 354, 64: 340, 128: 611}),
+    ("ct mc", (128, 128, 128), "f32", (16, 8), 353, {4: 357, 6: 324, 8: 308, 12: 306, 16: 326, 24: 326, 32: 403, 64: 376, 128: 656}),
+    ("unsplit mc", (128, 64, 96), "f32", (32, 4), 225, {4: 164, 6: 162, 8: 149, 12: 186, 16: 142, 24: 159, 32: 209, 48: 294, 64: 388}),
+    ("unsplit mc", (256, 256, 256), "f32", (16, 8), 2249, {4: 3133, 6: 2816, 8: 2647, 12: 2462, 16: 2325, 24: 2192, 32: 2194, 64: 2166, 128: 2509}),
+    ("unsplit mc", (64, 64, 64), "f64", (8, 8), 506, {4: 401, 6: 385, 8: 499, 12: 380, 16: 491, 24: 726, 32: 949, 64: 1806}),
+    ("unsplit mc", (128, 64, 96), "f64", (8, 8), 1004, {4: 952, 6: 975, 8: 1019, 12: 1114, 16: 996, 24: 1425, 32: 990, 64: 1930, 96: 2792}),
+    ("ct mc", (128, 128, 128), "f64", (8, 8), 2999, {4: 3262, 6: 3140, 8: 3133, 12: 3115, 16: 3052, 24: 3167, 32: 3382, 64: 3403, 128: 3380}),
+]
+
+
+@pytest.mark.parametrize("what,n,dtype,tile,before,times", CHUNK_TIMES)
+def test_chunks_are_no_slower_than_eight_rounds_of_blocks(plan, what, n, dtype, tile, before, times):
+    """The planes per block that the rule takes were measured no slower than what it replaced (2 %: two runs)."""
+    cols = -(-n[0] // tile[0]) * -(-n[1] // tile[1])
+    (lz,), = plan(("chunk", cols, n[2], 8 if dtype == "f64" else 4, tile[0] * tile[1]))
+    assert lz in times, lz
+    assert times[lz] <= 1.02 * before
+
+
 def test_scratch_is_handed_on_however_a_holder_leaves(tmp_path):
     """ScratchTurn (gmt_turn.h) over stand-ins of the runtime calls (tests/host/turn.cpp): a holder that leaves
     by an error exit after launching has its work marked like any other; one that could not wait for the last
