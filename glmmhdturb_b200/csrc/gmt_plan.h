@@ -54,12 +54,15 @@ inline int choose_chunk(long cols, int nz, int esize, int threads) {
         return (int)lz;
     }
     // a block takes lz planes and 2.8 planes' time for its start and for the first and last planes, which
-    // only reconstruct (64^3, chunk 4 -> 64: 41 -> 401 us, 6.05 us a plane)
+    // only reconstruct (FP32, 64^3, chunk 4 -> 64: 41 -> 401 us, 6.05 us a plane).  In FP64 a plane is mostly
+    // its Riemann solves, which those planes do without: 0.4 to 1.2 planes (chunk sweeps of the march and CT, MC
+    // and PPM, 64^3 to 160^3), and no share for the last round.  At 2.8 planes 128^3 got chunks of half the box
+    // or all of it where 8 and 16 planes are faster: march PPM 2733 -> 2554 us, CT PPM 5802 -> 5306 us.
     // Four planes at least.  Shorter chunks finish a small box that has the chip to itself sooner (32^3:
     // 20 us at 1, 33 at 3, 39 at 4; 48^3: 29 at 2, 41 at 4; with one chunk a tile 64 and 46), but more than
     // 40 % of each block is then its start.  Looping over single boxes is to stay at no more than half of the
     // ensemble's rate, which the loop's small boxes at 1 or 2 planes broke (5.65 against 11.2 Gzone/s; now 5.26).
-    constexpr double start = 2.8;
+    const double start = esize == 8 ? 0.8 : 2.8, tail = esize == 8 ? 0.0 : 0.2;
     double best = 1e300;
     int last = 0, choice = nz;
     for (int nch = 1; nch <= std::min(nz, 4096); ++nch) {
@@ -67,7 +70,7 @@ inline int choose_chunk(long cols, int nz, int esize, int threads) {
         if (lz == last || (lz < 4 && nch > 1)) continue;
         last = lz;
         const long rounds = (cols * (((long)nz + lz - 1) / lz) + 147) / 148;
-        const double cost = ((double)rounds + (rounds > 1 ? 0.2 : 0.0)) * (lz + start);
+        const double cost = ((double)rounds + (rounds > 1 ? tail : 0.0)) * (lz + start);
         if (cost < best) { best = cost; choice = lz; }
     }
     return choice;

@@ -74,6 +74,22 @@ CHUNK_TIMES = [
     ("unsplit mc", (64, 64, 64), "f64", (8, 8), 506, {4: 401, 6: 385, 8: 499, 12: 380, 16: 491, 24: 726, 32: 949, 64: 1806}),
     ("unsplit mc", (128, 64, 96), "f64", (8, 8), 1004, {4: 952, 6: 975, 8: 1019, 12: 1114, 16: 996, 24: 1425, 32: 990, 64: 1930, 96: 2792}),
     ("ct mc", (128, 128, 128), "f64", (8, 8), 2999, {4: 3262, 6: 3140, 8: 3133, 12: 3115, 16: 3052, 24: 3167, 32: 3382, 64: 3403, 128: 3380}),
+    # one block fills an SM
+    ("unsplit mc", (128, 128, 128), "f64", (16, 16), 1725, {4: 1746, 6: 1718, 8: 1654, 12: 1711, 16: 1817, 24: 1981, 32: 1801, 64: 1779, 128: 3363}),
+    ("unsplit ppm", (128, 128, 128), "f64", (32, 8), 2985, {4: 3107, 6: 3046, 8: 2964, 12: 3065, 16: 3274, 24: 3554, 32: 3245, 64: 3166, 128: 6051}),
+    ("unsplit ppm", (128, 128, 128), "f64", (16, 8), 6062, {4: 6458, 6: 6243, 8: 6128, 12: 6140, 16: 5961, 24: 6275, 32: 6682, 64: 6661, 128: 6573}),
+    ("unsplit ppm", (128, 64, 96), "f64", (16, 16), 1240, {4: 1244, 6: 1219, 8: 1200, 11: 1091, 12: 1181, 16: 1531, 24: 1142, 32: 1471, 64: 2897}),
+    ("unsplit mc", (128, 64, 96), "f64", (16, 8), 1358, {4: 1437, 6: 1337, 8: 1441, 11: 1326, 12: 1446, 16: 1442, 24: 1429, 32: 1846, 48: 1398, 64: 1831}),
+    ("march1d mc", (128, 128, 128), "f64", (16, 8), 1451, {4: 1656, 6: 1536, 8: 1485, 12: 1439, 16: 1426, 24: 1405, 32: 1485, 64: 1479, 128: 1533}),
+    ("ct mc", (128, 64, 96), "f64", (16, 8), 1139, {4: 1202, 6: 1144, 8: 1229, 11: 1130, 12: 1231, 16: 1239, 24: 1230, 32: 1573, 48: 1216, 64: 1581}),
+    ("ct mc", (64, 64, 64), "f64", (16, 8), 420, {4: 439, 6: 465, 8: 425, 12: 568, 16: 408, 24: 576, 32: 740, 64: 1491}),
+    ("march1d ppm", (128, 128, 128), "f64", (16, 16), 2569, {4: 2683, 8: 2554, 10: 2622, 12: 2638, 16: 2802, 20: 2637, 24: 3017, 32: 2796, 40: 3375, 48: 3292, 64: 2734, 80: 3340}),
+    ("march1d mc", (96, 96, 96), "f64", (16, 16), 366, {4: 380, 8: 339, 10: 399, 12: 327, 16: 413, 20: 454, 24: 316, 32: 408, 40: 502}),
+    ("march1d ppm", (160, 160, 160), "f64", (16, 16), 4970, {4: 5187, 8: 5069, 10: 4957, 12: 4883, 16: 4969, 20: 5234, 24: 5015, 32: 5542, 40: 5215, 48: 5898, 64: 5511, 80: 6854, 128: 5514}),
+    ("ct mc", (128, 128, 128), "f64", (16, 8), 3039, {4: 3056, 8: 2924, 10: 2956, 12: 2909, 16: 2857, 20: 2944, 24: 2989, 32: 3201, 40: 3007, 48: 3175, 64: 3192, 80: 3184, 128: 3146}),
+    ("ct ppm", (128, 128, 128), "f64", (16, 8), 5595, {4: 5657, 8: 5425, 10: 5498, 12: 5393, 16: 5306, 20: 5472, 24: 5547, 32: 5924, 40: 5580, 48: 5875, 64: 5922, 80: 5909, 128: 5800}),
+    ("ct mc", (112, 112, 112), "f64", (16, 8), 2043, {4: 2082, 8: 2072, 10: 2049, 12: 1956, 16: 2039, 20: 2012, 24: 2049, 32: 2023, 38: 1903, 40: 1986, 48: 2358, 64: 2398, 80: 2015}),
+    ("ct mc", (144, 144, 144), "f64", (16, 8), 4141, {4: 4311, 8: 4154, 10: 4075, 12: 4145, 16: 4090, 20: 4053, 24: 4229, 32: 4044, 40: 4210, 48: 4713, 64: 4628, 80: 5054, 128: 5989}),
 ]
 
 
