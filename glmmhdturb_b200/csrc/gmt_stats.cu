@@ -32,7 +32,8 @@ __global__ void __launch_bounds__(256) twiddle_kernel(int nx, int ny, int nz, in
 
 // Stage x: A[c][kx][row] = sum_x w_c(x,row) e^{-i 2pi kx x/nx}, row = y + ny z.
 // A block takes 32 rows.  Chunks of 32 columns are staged through shared memory, where w = m/sqrt(rho)
-// is formed once per cell (one reciprocal root for the three components); lane l of every warp then
+// is formed once per cell (one reciprocal root for the three components: 256^3 call 589 us, with a root and three
+// divisions 672 us, and the error of E against exact arithmetic the same, 3.92 and 3.91 x 2^-53 at worst); lane l of every warp then
 // owns row l, and warp g accumulates the SX_K wavenumbers g SX_K .. of all three components in
 // registers, so a staged value feeds 2 SX_K FMAs and the twiddles are warp-uniform (broadcast) reads.
 // Bound by the FP64 pipes: 6 (kmax+1) FMAs and a root per cell.  256^3 FP32, kmax = 8: 3.56 ms for one
