@@ -656,9 +656,14 @@ int gmt_kernel_info(gmt_ctx* c, int32_t* regs, int64_t* smem, int32_t tile[3]) {
     if (!c) return fail(GMT_ERR_ARG, "null context");
     int r = -1;
     int64_t sm = 0;
-    if (c->p.scheme == GMT_SCHEME_UNSPLIT) {
-        r = unsplit_regs(c->esize, c->p.recon, c->p.riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : c->p.riemann,
-                         c->ox * c->oy);
+    int t[3] = {c->ox, c->oy, c->lz};
+    const int riem = c->p.riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : c->p.riemann;
+    if (c->pass) {
+        r = passes_regs(c->p.recon, riem);
+        sm = (int64_t)passes_smem();
+        t[0] = PASS_TX; t[1] = PASS_TY; t[2] = pass_flux_planes(c->p.nx, c->p.ny, c->pass_S);
+    } else if (c->p.scheme == GMT_SCHEME_UNSPLIT) {
+        r = unsplit_regs(c->esize, c->p.recon, riem, c->ox * c->oy);
         sm = (int64_t)unsplit_smem(c->esize, c->ox, c->oy);
     } else if (c->p.scheme == GMT_SCHEME_MARCH1D) {
         r = c->esize == 8 ? march_tiled_regs((const UnsplitArgs<double>*)nullptr, c->p.recon, c->ox * c->oy)
@@ -670,7 +675,7 @@ int gmt_kernel_info(gmt_ctx* c, int32_t* regs, int64_t* smem, int32_t tile[3]) {
     }
     if (regs) *regs = r;
     if (smem) *smem = sm;
-    if (tile) { tile[0] = c->ox; tile[1] = c->oy; tile[2] = c->lz; }
+    if (tile) std::copy(t, t + 3, tile);
     return GMT_OK;
 }
 

@@ -17,6 +17,8 @@ cudaError_t launch_unsplit(const UnsplitArgs<float>& A, int recon, int riem, cud
 cudaError_t launch_unsplit(const UnsplitArgs<double>& A, int recon, int riem, cudaStream_t s);
 // the FP64 step as three passes over z slabs of S planes with caller-supplied scratch
 cudaError_t launch_passes(const UnsplitArgs<double>& A, int recon, int riem, void* scratch, int S, cudaStream_t s);
+int passes_regs(int recon, int riem);
+size_t passes_smem();
 int unsplit_max_threads(int dtype_bytes);
 cudaError_t unsplit_prepare_f32();   // shared-memory attributes of every step kernel
 cudaError_t unsplit_prepare_f64();

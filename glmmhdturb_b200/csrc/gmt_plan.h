@@ -7,6 +7,7 @@ namespace gmt {
 
 // --- the FP64 step's passes (gmt_passes.cuh) -----------------------------------------------------
 constexpr int PASS_TX = 16, PASS_TY = 8;   // columns per block of the flux pass
+constexpr int PASS_MINB = 4;               // its blocks on an SM
 constexpr size_t PASS_SCRATCH_BYTES = (size_t)1 << 30;   // of a context, or of all lanes of an ensemble
 constexpr int GRID_YZ = 65535;             // largest gridDim.y and gridDim.z
 
@@ -29,6 +30,15 @@ inline int pass_slab(int nx, int ny, int nz, size_t budget) {
     auto over = [&] { return passes_scratch_bytes(nx, ny, planes()) > budget; };
     while (planes() > GRID_YZ - 4 || (planes() > 4 && over())) ++slabs;
     return over() ? 0 : planes();
+}
+
+// planes per block of the flux pass over a slab of S planes: the extra z face of a chunk costs a third of a
+// plane, so long chunks, but enough blocks for several rounds of PASS_MINB blocks on every SM
+inline int pass_flux_planes(int nx, int ny, int S) {
+    const long bx = (nx + PASS_TX - 1) / PASS_TX, by = (ny + PASS_TY - 1) / PASS_TY;
+    int lz = S;
+    while (lz > 4 && bx * by * ((S + lz - 1) / lz) < 148L * PASS_MINB * 3) lz = (lz + 1) / 2;
+    return lz;
 }
 
 // --- z chunks of the tile marches ----------------------------------------------------------------

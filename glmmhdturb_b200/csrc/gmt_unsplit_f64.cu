@@ -23,7 +23,7 @@ cudaError_t launch_unsplit(const UnsplitArgs<double>& A, int recon, int riem, cu
     return unsplit_dispatch_t<double, 256, 1>(A, recon, riem, s);
 }
 // The step as three passes over z slabs of S planes (gmt_passes.cuh); scratch of passes_scratch_bytes.
-constexpr int PTX = PASS_TX, PTY = PASS_TY, PMINB = 4;
+constexpr int PTX = PASS_TX, PTY = PASS_TY, PMINB = PASS_MINB;
 template <int RECON, int RIEM>
 static cudaError_t passes_go(const UnsplitArgs<double>& A, void* scratch, int S, cudaStream_t s) {
     const size_t nxy = (size_t)A.nx * A.ny;
@@ -39,11 +39,7 @@ static cudaError_t passes_go(const UnsplitArgs<double>& A, void* scratch, int S,
         pass_recon_kernel<double, RECON><<<dim3((unsigned)((nxy + 127) / 128), P.S + 2), 128, 0, s>>>(P);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;   // no fluxes from scratch that was not written
-        // planes per block of the flux pass: the extra z face of a chunk costs a third of a plane, so
-        // long chunks, but enough blocks for several rounds of PMINB blocks on every SM
-        int lz = P.S;
-        while (lz > 4 && (long)bx * by * ((P.S + lz - 1) / lz) < 148L * PMINB * 3) lz = (lz + 1) / 2;
-        P.lz = lz;
+        const int lz = P.lz = pass_flux_planes(A.nx, A.ny, P.S);
         pass_flux_kernel<double, RECON, RIEM, PTX, PTY, PMINB>
             <<<dim3(bx, by, (P.S + lz - 1) / lz), PTX * PTY, pass_flux_smem<PTX, PTY>(sizeof(double)), s>>>(P);
     }
@@ -58,6 +54,19 @@ cudaError_t launch_passes(const UnsplitArgs<double>& A, int recon, int riem, voi
 #undef GMT_CASE
     return cudaErrorInvalidValue;
 }
+// registers and dynamic shared memory of the flux pass, the step's longest
+int passes_regs(int recon, int riem) {
+    cudaFuncAttributes fa{};
+    cudaError_t e = cudaErrorInvalidValue;
+#define GMT_CASE(RC, RM) \
+    if (recon == RC && riem == RM) e = cudaFuncGetAttributes(&fa, pass_flux_kernel<double, RC, RM, PTX, PTY, PMINB>);
+    GMT_CASE(RECON_MC, RIEM_HLLD) GMT_CASE(RECON_MC, RIEM_HLL) GMT_CASE(RECON_MC, RIEM_LLF_BOUND)
+    GMT_CASE(RECON_MINMOD, RIEM_HLLD) GMT_CASE(RECON_MINMOD, RIEM_HLL) GMT_CASE(RECON_MINMOD, RIEM_LLF_BOUND)
+    GMT_CASE(RECON_PPM, RIEM_HLLD) GMT_CASE(RECON_PPM, RIEM_HLL) GMT_CASE(RECON_PPM, RIEM_LLF_BOUND)
+#undef GMT_CASE
+    return e == cudaSuccess ? fa.numRegs : -1;
+}
+size_t passes_smem() { return pass_flux_smem<PTX, PTY>(sizeof(double)); }
 cudaError_t unsplit_prepare_f64() {
     cudaError_t e = unsplit_configure_all_t<double, 256, 1>();
 #define GMT_FIX(RC, RM)                                                                          \

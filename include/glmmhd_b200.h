@@ -103,7 +103,8 @@ int gmt_params_init(gmt_params* p, int n);
  * where a cross section needs more, the step runs as the tile march, with the same bits) */
 int gmt_create(const gmt_params* p, gmt_ctx** out);
 int gmt_destroy(gmt_ctx* ctx);
-/* kernel resource report: registers, dynamic shared bytes and tile of the step kernel */
+/* kernel resource report: registers, dynamic shared bytes and tile of the step kernel (of the flux pass
+ * where the FP64 unsplit step runs as passes) */
 int gmt_kernel_info(gmt_ctx* ctx, int32_t* regs, int64_t* smem_bytes, int32_t tile[3]);
 
 /* --- GLM step (unsplit: step_plm!/step_tiled!/step_multi!; march1d: march_run_dev) ------- */

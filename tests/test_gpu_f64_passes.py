@@ -58,6 +58,16 @@ def test_more_planes_than_a_launch_takes():
     assert a.cfl_result() == b.cfl_result()
 
 
+def test_kernel_info_reports_the_route():
+    """The flux pass of a context that runs the passes (16x8 columns, 128 registers for four blocks per SM, its
+    shared memory below the 48 KB of a launch without attributes); the march of one whose tile was chosen."""
+    from glmmhdturb_b200 import Solver
+    a = Solver((48, 32, 13), dtype="f64").kernel_info()
+    b = Solver((48, 32, 13), dtype="f64", tile=(16, 16, 0)).kernel_info()
+    assert a["tile"][:2] == (16, 8) and 1 <= a["tile"][2] <= 13 and 0 < a["regs"] <= 128 and 0 < a["smem"] <= 48 * 1024
+    assert b["tile"][:2] == (16, 16) and b["regs"] > 128 and b["smem"] > 48 * 1024
+
+
 def test_under_capture_and_after():
     """A captured step takes the tile march (it must not be ordered against work outside its graph)."""
     from glmmhdturb_b200 import Solver
