@@ -6,11 +6,11 @@
 
 namespace gmt {
 // compile-time tiles for the production schemes (PLM-MC / PPM with HLLD / HLL)
-template <int TOX, int TOY, int MAXT = 512, int MINB = 1>
+template <int TOX, int TOY, int MAXT = 512, int MINB = 1, bool MAY_OVER = false>
 static bool fixed_tile(const UnsplitArgs<float>& A, int recon, int riem, cudaStream_t s, cudaError_t& e) {
     if (A.ox != TOX || A.oy != TOY) return false;
 #define GMT_FIX(RC, RM) \
-    if (recon == RC && riem == RM) { e = unsplit_go<float, RC, RM, MAXT, MINB, TOX, TOY>(A, s); return true; }
+    if (recon == RC && riem == RM) { e = unsplit_go<float, RC, RM, MAXT, MINB, TOX, TOY, MAY_OVER>(A, s); return true; }
     GMT_FIX(RECON_MC, RIEM_HLLD) GMT_FIX(RECON_MC, RIEM_HLL) GMT_FIX(RECON_PPM, RIEM_HLLD) GMT_FIX(RECON_PPM, RIEM_HLL)
 #undef GMT_FIX
     return false;
@@ -18,7 +18,7 @@ static bool fixed_tile(const UnsplitArgs<float>& A, int recon, int riem, cudaStr
 
 cudaError_t launch_unsplit(const UnsplitArgs<float>& A, int recon, int riem, cudaStream_t s) {
     cudaError_t e = cudaSuccess;
-    if (fixed_tile<32, 16>(A, recon, riem, s, e) || fixed_tile<64, 8>(A, recon, riem, s, e) ||
+    if (fixed_tile<32, 16, 512, 1, true>(A, recon, riem, s, e) || fixed_tile<64, 8>(A, recon, riem, s, e) ||
         fixed_tile<16, 16, 256, 2>(A, recon, riem, s, e))
         return e;
     if (A.ox * A.oy > 256) return unsplit_dispatch_t<float, 512, 1>(A, recon, riem, s);
@@ -27,10 +27,10 @@ cudaError_t launch_unsplit(const UnsplitArgs<float>& A, int recon, int riem, cud
 cudaError_t unsplit_prepare_f32() {
     cudaError_t e = unsplit_configure_all_t<float, 256, 2>();
     if (e == cudaSuccess) e = unsplit_configure_all_t<float, 512, 1>();
-#define GMT_FIX(RC, RM)                                                              \
-    if (e == cudaSuccess) e = unsplit_configure<float, RC, RM, 512, 1, 32, 16>();    \
-    if (e == cudaSuccess) e = unsplit_configure<float, RC, RM, 512, 1, 64, 8>();     \
-    if (e == cudaSuccess) e = unsplit_configure<float, RC, RM, 256, 2, 16, 16>();
+#define GMT_FIX(RC, RM)                                                                  \
+    if (e == cudaSuccess) e = unsplit_configure<float, RC, RM, 512, 1, 32, 16>();        \
+    if (e == cudaSuccess) e = unsplit_configure<float, RC, RM, 512, 1, 64, 8, false>();  \
+    if (e == cudaSuccess) e = unsplit_configure<float, RC, RM, 256, 2, 16, 16, false>();
     GMT_FIX(RECON_MC, RIEM_HLLD) GMT_FIX(RECON_MC, RIEM_HLL) GMT_FIX(RECON_PPM, RIEM_HLLD) GMT_FIX(RECON_PPM, RIEM_HLL)
 #undef GMT_FIX
     UnsplitArgs<float> none{};

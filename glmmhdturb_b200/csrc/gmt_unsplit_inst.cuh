@@ -46,15 +46,21 @@ static cudaError_t unsplit_run(const UnsplitArgs<R>* A, cudaStream_t s, bool con
     return cudaGetLastError();
 }
 template <class R> inline bool overhangs(const UnsplitArgs<R>& A) { return A.nx % A.ox != 0 || A.ny % A.oy != 0; }
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
+// MAY_OVER: the tile is one that the library chooses for boxes that it does not divide; tiles that only a caller
+// chooses, and 16x16 of an FP32 ensemble, whose boxes are multiples of 16, have no overhanging kernel
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0, bool MAY_OVER = true>
 static cudaError_t unsplit_configure() {
-    cudaError_t e = unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, true>(nullptr, 0, true);
+    cudaError_t e = cudaSuccess;
+    if constexpr (MAY_OVER) e = unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, true>(nullptr, 0, true);
     if (e == cudaSuccess && TOX > 0) e = unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, TOX == 0>(nullptr, 0, true);
     return e;
 }
-template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0>
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX = 0, int TOY = 0, bool MAY_OVER = true>
 static cudaError_t unsplit_go(const UnsplitArgs<R>& A, cudaStream_t s) {
-    if (TOX == 0 || overhangs(A)) return unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, true>(&A, s, false);
+    if (TOX == 0 || overhangs(A)) {
+        if constexpr (MAY_OVER) return unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, true>(&A, s, false);
+        else return cudaErrorInvalidConfiguration;
+    }
     return unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, TOX == 0>(&A, s, false);
 }
 
