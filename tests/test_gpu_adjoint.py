@@ -91,6 +91,30 @@ def test_one_step_adjoint_vs_oracle_forward_mode(oracle, recon, riemann):
     assert abs(amp_part - fwd_amp) <= DOT_TOL * float(np.abs(w * ja).sum()) / 2.0, (amp_part, fwd_amp)
 
 
+@pytest.mark.parametrize("n,recon,riemann", [((9, 14, 5), "mc", "hlld"), ((33, 6, 7), "minmod", "hll"), ((3, 1, 4), "mc", "hlld")])
+def test_one_step_adjoint_on_odd_grids(oracle, n, recon, riemann):
+    """The FP64 passes from primitive planes on uneven boxes, also with axes shorter than a stencil, against the
+    oracle's forward-mode tangents (as above)."""
+    u0 = perturbed_glm_state(oracle, n, seed=12, gamma=GAMMA)
+    cfg = oracle.Config(n=n, gamma=GAMMA, recon=recon, riemann=riemann, iflo=True)
+    s = _solver(n, recon=recon, riemann=riemann)
+    s.forcing_reset()
+    s.forcing_advance()
+    cmax, ch = oracle.cfl(cfg, u0)
+    dt = 0.3 * cfg.dx / cmax
+    fac = math.exp(-(ch / 0.18) * dt)
+    rng = np.random.default_rng(8)
+    w = rng.standard_normal(u0.shape)
+    gin = torch.full_like(to_dev(u0), float("nan"))
+    s.adjoint_step(to_dev(u0), to_dev(w), gin, dt, t=0.2, ch=ch, glm_fac=fac, do_turb=True)
+    jtw = gin.cpu().numpy()
+    v = rng.standard_normal((4,) + u0.shape) * np.abs(u0).max(axis=(1, 2, 3), keepdims=True)
+    _, jv = oracle.jvp_unsplit(cfg, u0, v, dt, ch, fac, ramp=0.4, modes=s.get_modes())
+    for k in range(4):
+        lhs, rhs = float((w * jv[k]).sum()), float((jtw * v[k]).sum())
+        assert abs(lhs - rhs) <= DOT_TOL * float(np.abs(w * jv[k]).sum()), (k, lhs, rhs)
+
+
 def _scaled(sched, f):
     import copy
     s2 = copy.copy(sched)

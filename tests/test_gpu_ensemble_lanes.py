@@ -1,0 +1,64 @@
+"""Ensembles whose boxes share a stream (more boxes than lanes: 64 in FP32, 4 in FP64, where a lane's boxes also
+take its scratch in turn), runs without and with the replayed pair of steps, odd and even numbers of
+steps, and a box of several slabs.  Every box must equal its own single-box run."""
+import pytest
+import torch
+
+from tests.gpu_util import max_rel_err
+
+pytestmark = pytest.mark.gpu
+
+COURANT, CP, T = 0.3, 0.18, 0.5
+
+
+def _runs(sizes, dtype, steps, graph=True):
+    """The ensemble's states and times after `steps` steps, and each box's from a single-box run."""
+    from glmmhdturb_b200 import Ensemble, Solver
+    amps, seeds = [1.0 + 0.25 * (b % 7) for b in range(len(sizes))], [11 + b for b in range(len(sizes))]
+    ens = Ensemble(sizes, amps=amps, seeds=seeds, dtype=dtype, courant=COURANT, turb_T=T, glm_cp_coef=CP)
+    u, w = ens.alloc(), ens.alloc()
+    singles = []
+    for b, n in enumerate(sizes):
+        s = Solver(n, dtype=dtype, gamma=5 / 3, courant=COURANT, turb_amp=amps[b], turb_T=T, turb_ndt=100, turb_seed=seeds[b],
+                   glm_cp_coef=CP)
+        s.ic_turbulent(u[b], mach=0.5 + 0.1 * (b % 6), seed=seeds[b])
+        x, y = u[b].clone(), torch.empty_like(u[b])
+        s.forcing_reset()
+        singles.append(s.run(x, y, steps, forcing=True))
+        s.close()
+    t = ens.run(u, w, steps, forcing=True, graph=graph)
+    return t, (w if steps % 2 else u), singles
+
+
+@pytest.mark.parametrize("steps", [3, 6])
+def test_fp64_boxes_share_lanes_and_their_scratch(steps):
+    """Eight uneven boxes on four lanes; the mean box is below the size from which steps are not replayed."""
+    t, got, singles = _runs([32, 48, 16, 64, 32, 16, 48, 32], "f64", steps)
+    for b, (ts, ref) in enumerate(singles):
+        assert t[b] == ts and torch.equal(got[b], ref), b
+
+
+def test_fp64_box_of_several_slabs_beside_others():
+    """With four lanes a 144^3 box has two slabs; the mean box is above 48^3, so no steps are replayed."""
+    t, got, singles = _runs([144, 64, 80, 96, 32], "f64", 3)
+    for b, (ts, ref) in enumerate(singles):
+        assert t[b] == ts and torch.equal(got[b], ref), b
+
+
+def _check_f32(t, got, singles):
+    for b, (ts, ref) in enumerate(singles):
+        assert abs(t[b] - ts) <= 1e-6 * ts
+        # other tiles than the single box's: FP32 round-off (1e-7..6e-7 after nine steps; psi, small, up to 6e-5)
+        err, errs = max_rel_err(got[b].cpu().numpy(), ref.cpu().numpy())
+        assert max(errs[:8]) <= 1e-5 and errs[8] <= 1e-3, (b, errs)
+
+
+@pytest.mark.parametrize("steps", [4, 5])
+def test_fp32_steps_that_are_not_replayed(steps):
+    """A mean box above 48^3 takes plain launches, whether or not a graph is asked for."""
+    _check_f32(*_runs([64, 48, 96, 64], "f32", steps))
+
+
+@pytest.mark.parametrize("steps,graph", [(4, True), (5, True), (5, False)])
+def test_fp32_more_boxes_than_lanes(steps, graph):
+    _check_f32(*_runs([16, 32, 16, 48, 16] * 14, "f32", steps, graph))
