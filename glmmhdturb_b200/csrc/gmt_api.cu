@@ -76,8 +76,9 @@ double forcing_sigma0(double amp, double alpha, double beta) {
 // leaves idle (64 uneven boxes, 41 M zones: 4.22 ms a step over 8 streams, 3.83 over 32, 3.65 over 64).
 // The single-box kernels run here, with a box's arguments in constant memory: a persistent kernel over
 // a queue of tiles of all boxes held them in registers, spilled, and took 3.95 ms.
-// In FP64 every lane has the passes' scratch of the largest box, an equal share of a context's at most.
-constexpr int ENS_LANES = 64, ENS_LANES_F64 = 4;
+// In FP64 (pass_lanes) every lane has the passes' scratch of the largest box, an equal share of a context's at
+// most.
+constexpr int ENS_LANES = 64;
 // Mean box below which two steps are replayed as a graph: a box's three launches take the host 7 us, about
 // what a 48^3 box takes the chip (64 boxes); above that plain launches keep the boxes' order, which the
 // graph's branches do not (41 M zones: 3.65 ms a step against 3.75 to 3.93).
@@ -1434,7 +1435,7 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
     }
 
     ens_tiles(E);
-    const int lanes = std::min(nbox, E->esize == 8 ? ENS_LANES_F64 : ENS_LANES);
+    const int lanes = E->esize == 8 ? pass_lanes(nbox, *std::max_element(n, n + nbox)) : std::min(nbox, ENS_LANES);
     E->lane.assign(lanes, nullptr);
     E->lane_ev.assign(lanes, nullptr);
     for (int i = 0; i < lanes; ++i) {

@@ -32,6 +32,15 @@ inline int pass_slab(int nx, int ny, int nz, size_t budget) {
     return over() ? 0 : planes();
 }
 
+// Lanes (streams with scratch of their own) of an FP64 ensemble: four, or two where a fourth of the budget
+// would cut the largest box into slabs.  ms a step with 1, 2, 4, 8, 16 lanes: 16 boxes of 32^3 1.59, 0.86,
+// 0.52, 0.40, 0.39; 8 of 96^3 3.80, 3.49, 3.54, 3.55, 3.56; cut into slabs from four lanes on, 6 of 128^3 6.57,
+// 6.09, 6.32, 6.33, 6.34, and 4 of 192^3 13.96, 13.58, 14.07, 14.08, 14.09 (two slabs with two lanes).
+inline int pass_lanes(int nbox, int largest) {
+    const int lanes = std::min(nbox, 4);
+    return passes_scratch_bytes(largest, largest, largest) <= PASS_SCRATCH_BYTES / lanes ? lanes : std::min(nbox, 2);
+}
+
 // planes per block of the flux pass over a slab of S planes: the extra z face of a chunk costs a third of a
 // plane, so long chunks, but enough blocks for several rounds of PASS_MINB blocks on every SM
 inline int pass_flux_planes(int nx, int ny, int S) {

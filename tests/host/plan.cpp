@@ -1,5 +1,6 @@
 // Prints what the rules of gmt_plan.h choose.  One query per line of standard input, one answer per line:
 //   slab nx ny nz lanes -> planes per slab of the FP64 passes of one of `lanes` lanes, bytes of their scratch
+//   lanes nbox largest -> lanes of an FP64 ensemble
 //   chunk cols nz esize threads -> planes per block of a tile march
 #include <cstdio>
 #include <cstring>
@@ -14,6 +15,10 @@ int main() {
             if (std::scanf("%d %d %d %d", &nx, &ny, &nz, &lanes) != 4) return 1;
             const int S = gmt::pass_slab(nx, ny, nz, gmt::PASS_SCRATCH_BYTES / lanes);
             std::printf("%d %zu\n", S, S > 0 ? gmt::passes_scratch_bytes(nx, ny, S) : (size_t)0);
+        } else if (!std::strcmp(what, "lanes")) {
+            int nbox, largest;
+            if (std::scanf("%d %d", &nbox, &largest) != 2) return 1;
+            std::printf("%d\n", gmt::pass_lanes(nbox, largest));
         } else if (!std::strcmp(what, "chunk")) {
             long cols;
             int nz, esize, threads;

@@ -1,4 +1,4 @@
-"""Ensembles whose boxes share a stream (more boxes than lanes: 64 in FP32, 4 in FP64, where a lane's boxes also
+"""Ensembles whose boxes share a stream (more boxes than lanes: 64 in FP32, 4 or 2 in FP64, where a lane's boxes also
 take its scratch in turn), runs without and with the replayed pair of steps, odd and even numbers of
 steps, and a box of several slabs.  Every box must equal its own single-box run."""
 import pytest
@@ -39,8 +39,8 @@ def test_fp64_boxes_share_lanes_and_their_scratch(steps):
 
 
 def test_fp64_box_of_several_slabs_beside_others():
-    """With four lanes a 144^3 box has two slabs; the mean box is above 48^3, so no steps are replayed."""
-    t, got, singles = _runs([144, 64, 80, 96, 32], "f64", 3)
+    """On two lanes a 160^3 box has two slabs; the mean box is above 48^3, so no steps are replayed."""
+    t, got, singles = _runs([160, 64, 80, 96, 32], "f64", 3)
     for b, (ts, ref) in enumerate(singles):
         assert t[b] == ts and torch.equal(got[b], ref), b
 

@@ -58,6 +58,13 @@ def test_fp64_scratch_stays_within_its_budget(plan, n, lanes):
         assert S >= min(3, n[2]) and size <= budget
 
 
+@pytest.mark.parametrize("nbox,largest,lanes", [(1, 192, 1), (2, 256, 2), (3, 128, 3), (4, 112, 4), (64, 32, 4), (4, 128, 2),
+                                                (64, 192, 2), (5, 512, 2)])
+def test_fp64_lanes_keep_boxes_whole_where_two_of_them_can(plan, nbox, largest, lanes):
+    (got,), = plan(("lanes", nbox, largest))
+    assert got == lanes
+
+
 # us a step of a tile march: with the rule that asked for eight rounds of blocks and no more (the kernels of
 # that time), and by planes per block.  Tiles of which several blocks share an SM:
 CHUNK_TIMES = [
