@@ -12,6 +12,7 @@
 #include "gmt_internal.h"
 #include "gmt_unsplit.cuh"
 #include "gmt_loop.cuh"
+#include "gmt_recent.h"
 #include "gmt_turn.h"
 
 using namespace gmt;
@@ -124,15 +125,18 @@ struct gmt_ctx {
     int adj_percell = 0;           // 1: the adjoint runs its first three passes per cell
     long long wait_cycles = GMT_WAIT_CYCLES;   // budget of the tile kernels' bounded waits
     int wait_test = 0;             // failure-path tests: staging withheld, so every bounded wait runs out
-    struct TmaMap { const void* base; int ox, oy; CUtensorMap map; };
-    TmaMap tma[4] = {};            // tensor maps of the last input states and tiles (tile staging)
-    int tma_next = 0;
-    struct CtTmaMap { const void* base; CUtensorMap map8, map1; };
-    CtTmaMap ct_tma[2] = {};       // the same for the CT state (8 variables, and bzf alone)
-    int ct_tma_next = 0;
+    // tensor maps of the last input states and tiles (tile staging); of a CT state the 8 variables, and bzf alone
+    struct TileOf {
+        const void* base;
+        int ox, oy;
+        bool operator==(const TileOf& o) const { return base == o.base && ox == o.ox && oy == o.oy; }
+    };
+    struct CtMaps { CUtensorMap map8, map1; };
+    Recent<TileOf, CUtensorMap, 4> tma;
+    Recent<TileOf, CtMaps, 2> ct_tma;
     // scratch of the FP64 step's passes (slabs of pass_S planes; null: the tile march).  Steps of one
     // context on several streams or threads take it in turn (ScratchTurn).  It alone is shared so: the CFL
-    // words, the forcing and loop records and the tensor maps are the caller's to keep apart.
+    // words, the forcing and loop records and the scratch of CT and of species are the caller's to keep apart.
     void* pass = nullptr;
     int pass_S = 0;
     cudaEvent_t pass_ev = nullptr;
@@ -255,17 +259,13 @@ template <class R> bool set_staging(UnsplitArgs<R>& A) {
 }
 // the same with the context's maps of its last input states
 template <class R> void set_tma(gmt_ctx* c, UnsplitArgs<R>& A) {
-    const R* base = tma_base<R>(A.u, 9, A.nx, A.ny, A.nz, A.ox, A.oy, 4);
-    for (const gmt_ctx::TmaMap& t : c->tma)
-        if (base && t.base == base && t.ox == A.ox && t.oy == A.oy) {
-            A.quad = quad_ok<R>(A.u.p, 9, A.nx, A.ox);
-            A.tmap = t.map;
-            A.use_tma = 1;
-            return;
-        }
-    if (!set_staging(A)) return;
-    c->tma[c->tma_next] = {base, A.ox, A.oy, A.tmap};
-    c->tma_next = (c->tma_next + 1) & 3;
+    const gmt_ctx::TileOf key{tma_base<R>(A.u, 9, A.nx, A.ny, A.nz, A.ox, A.oy, 4), A.ox, A.oy};
+    if (key.base && c->tma.find(key, &A.tmap)) {
+        A.quad = quad_ok<R>(A.u.p, 9, A.nx, A.ox);
+        A.use_tma = 1;
+    } else if (set_staging(A)) {
+        c->tma.keep(key, A.tmap);
+    }
 }
 
 // CT: the staged region is (ox+8) x (oy+5) cells; one map moves the 8 state variables, one bzf
@@ -276,22 +276,15 @@ template <class R> void set_ct_tma(gmt_ctx* c, CTArgs<R>& A) {
     std::memset(&A.tmap1, 0, sizeof(A.tmap1));
     const R* base = tma_base<R>(A.q, 8, A.nx, A.ny, A.nz, A.ox, A.oy, 5);
     if (!base) return;
-    for (const gmt_ctx::CtTmaMap& t : c->ct_tma)
-        if (t.base == base) {
-            A.tmap8 = t.map8;
-            A.tmap1 = t.map1;
-            A.use_tma = 1;
-            return;
-        }
-    CUtensorMap m8, m1;
-    if (!encode_state_map(&m8, base, A.nx, A.ny, A.nz, 8, A.ox + 8, A.oy + 5, 8)) return;
-    if (!encode_state_map(&m1, base, A.nx, A.ny, A.nz, 8, A.ox + 8, A.oy + 5, 1)) return;
-    c->ct_tma[c->ct_tma_next].base = base;
-    c->ct_tma[c->ct_tma_next].map8 = m8;
-    c->ct_tma[c->ct_tma_next].map1 = m1;
-    c->ct_tma_next ^= 1;
-    A.tmap8 = m8;
-    A.tmap1 = m1;
+    const gmt_ctx::TileOf key{base, A.ox, A.oy};
+    gmt_ctx::CtMaps m;
+    if (!c->ct_tma.find(key, &m)) {
+        if (!encode_state_map(&m.map8, base, A.nx, A.ny, A.nz, 8, A.ox + 8, A.oy + 5, 8)) return;
+        if (!encode_state_map(&m.map1, base, A.nx, A.ny, A.nz, 8, A.ox + 8, A.oy + 5, 1)) return;
+        c->ct_tma.keep(key, m);
+    }
+    A.tmap8 = m.map8;
+    A.tmap1 = m.map1;
     A.use_tma = 1;
 }
 

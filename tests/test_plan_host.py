@@ -1,5 +1,5 @@
 """Host code of the library without a GPU: the rules that cut a step up for its grid (gmt_plan.h; tests/host/plan.cpp
-prints their choices), and the turns at shared scratch (gmt_turn.h)."""
+prints their choices), the turns at shared scratch (gmt_turn.h), and what is kept for later steps (gmt_recent.h)."""
 import os
 import shutil
 import subprocess
@@ -127,3 +127,17 @@ def test_scratch_is_handed_on_however_a_holder_leaves(tmp_path):
     assert got[2] == ["wait 1", "status 1", "free 1"]
     assert got[3] == ["wait 1", "launch 1", "record 1", "synchronise 1", "status 1", "free 1"]
     assert got[4] == ["wait 1", "launch 1", "record 1", "wait 2", "launch 2", "record 2"]
+
+
+def test_tensor_maps_kept_for_later_steps_are_whole(tmp_path):
+    """What a context keeps of its last input states (gmt_recent.h), under threads that step on more states than
+    it holds: a map that another thread was writing would be handed to the TMA unit."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("no C++ compiler")
+    exe = str(tmp_path / "recent")
+    subprocess.run([cxx, "-std=c++17", "-O2", "-Wall", "-Werror", "-pthread", "-o", exe, os.path.join(HERE, "host", "recent.cpp")],
+                   check=True)
+    found, torn, oldest, rest = subprocess.run([exe], check=True, capture_output=True, text=True, timeout=120).stdout.split()
+    assert int(found) > 0 and int(torn) == 0
+    assert oldest == "0" and rest == "1111"
