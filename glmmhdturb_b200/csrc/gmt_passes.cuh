@@ -12,10 +12,11 @@
 // a small working set and enough warps in flight, for 18 planes of scratch written and read once
 // (slab-sized, so it is bounded and, for small boxes, stays in L2).  Every value is formed by the
 // expressions of the tile march in the same order, so the result is the same bit for bit.
-// MC + HLLD with forcing and CFL, tile march -> passes (192^3 with the one-body HLLD): 32^3 255 -> 94 us,
-// 64^3 258 -> 160 us, 192^3 6.1 -> 3.45 ms, 256^3 14.1 -> 8.6 ms.  At 192^3 the primitives take 0.15 ms (at
-// the memory's rate), the predictor 0.5 ms (FP64 pipes 53 % busy), the fluxes the rest, bound by dependent
-// FP64 chains and instruction fetch at 16 warps per SM.
+// MC + HLLD with forcing and CFL, tile march -> passes: 32^3 133 -> 87 us, 64^3 251 -> 141 us, 128^3 1.79 -> 1.02
+// ms, 192^3 5.83 -> 3.25 ms, 256^3 13.7 -> 8.0 ms, 512^3 110 -> 64.7 ms.  At 128^3 (profiled) the primitives take 44 us, at
+// 73 % of the memory's rate; the predictor 147 us at 12 warps per SM (MC's 168 registers), the busiest pipe 62 %
+// of its time; the fluxes 778 us at 16 warps per SM (128 registers, 56 bytes spilled; PPM 32 to 96), waiting for
+// fixed latencies, for one another at the barriers (24 threads solve a fourth face) and for instructions.
 #pragma once
 #include "gmt_unsplit.cuh"
 

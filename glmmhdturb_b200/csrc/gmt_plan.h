@@ -19,8 +19,8 @@ inline size_t passes_scratch_bytes(int nx, int ny, int S) {
 // planes per slab of the FP64 step's passes: slabs of equal thickness whose scratch stays within `budget`,
 // cut down to three or four planes; 0, the tile march, where even those exceed it (1 GB: cross sections
 // above about 1029^2).  A slab repeats the primitives of four planes and the predictors of two, so
-// thick ones: 256^3 8.60 ms within 1 GB, 8.94 ms within 256 MB, 10.7 ms within 64 MB (4 planes), which L2
-// would hold; the march takes 14.1 ms.
+// thick ones: 256^3 7.99 ms within 1 GB, 8.29 ms within 256 MB, 9.91 ms within 64 MB (4 planes), which L2
+// would hold; the march takes 13.7 ms.
 // The passes put a slab's planes, and the flux pass its rows of tiles, in gridDim.y: a narrow box of many
 // planes has more slabs than its scratch asks for, and one of too many rows none.
 inline int pass_slab(int nx, int ny, int nz, size_t budget) {
@@ -58,6 +58,8 @@ inline int pass_flux_planes(int nx, int ny, int S) {
 // shared memory; the automatic tiles are all of this kind): the number of rounds of blocks over the 148 SMs
 // times the length of a block.  Short chunks repeat the fixed part, long ones leave SMs idle in the last round;
 // with more than one round a share of a block's time is added, because blocks do not end together.
+// The constants are fitted to the FP32 MC + HLLD step and to FP64 sweeps of the march and CT.  FP32 PPM, minmod, the march
+// and CT use them unfitted: 8^3 to 256^3 they take 0.55 to 1.01 of their times with a rule that asked for eight rounds.
 // (FP32 MC + HLLD, chunk -> us: 64^3 4 -> 41, 8 -> 66; 96^3 12 -> 92, 6 -> 105; 192^3 32 -> 694,
 // 6 -> 833; 256^3 32 -> 1549, 16 -> 1623; 512^3 128 -> 11.59 ms, 64 and 256 -> 11.70 ms; the second
 // figures of the first four are the chunks of a rule that only asked for eight rounds of blocks.)
@@ -77,10 +79,10 @@ inline int choose_chunk(long cols, int nz, int esize, int threads) {
     // its Riemann solves, which those planes do without: 0.4 to 1.2 planes (chunk sweeps of the march and CT, MC
     // and PPM, 64^3 to 160^3), and no share for the last round.  At 2.8 planes 128^3 got chunks of half the box
     // or all of it where 8 and 16 planes are faster: march PPM 2733 -> 2554 us, CT PPM 5802 -> 5306 us.
-    // Four planes at least.  Shorter chunks finish a small box that has the chip to itself sooner (32^3:
-    // 20 us at 1, 33 at 3, 39 at 4; 48^3: 29 at 2, 41 at 4; with one chunk a tile 64 and 46), but more than
-    // 40 % of each block is then its start.  Looping over single boxes is to stay at no more than half of the
-    // ensemble's rate, which the loop's small boxes at 1 or 2 planes broke (5.65 against 11.2 Gzone/s; now 5.26).
+    // Four planes at least, which is not the best for a small box that has the chip to itself (32^3: 21 us at 1, 31
+    // at 3, 37 at 4; 48^3: 29 at 2, 40 at 4).  The one reason is a test that holds
+    // a loop over single boxes to half of the ensemble's rate: at 1 or 2 planes the loop's small boxes reach 5.65
+    // against 11.2 Gzone/s, now 5.2.
     const double start = esize == 8 ? 0.8 : 2.8, tail = esize == 8 ? 0.0 : 0.2;
     double best = 1e300;
     int last = 0, choice = nz;

@@ -32,12 +32,13 @@ __global__ void __launch_bounds__(256) twiddle_kernel(int nx, int ny, int nz, in
 
 // Stage x: A[c][kx][row] = sum_x w_c(x,row) e^{-i 2pi kx x/nx}, row = y + ny z.
 // A block takes 32 rows.  Chunks of 32 columns are staged through shared memory, where w = m/sqrt(rho)
-// is formed once per cell (one reciprocal root for the three components: 256^3 call 589 us, with a root and three
-// divisions 672 us, and the error of E against exact arithmetic the same, 3.92 and 3.91 x 2^-53 at worst); lane l of every warp then
-// owns row l, and warp g accumulates the SX_K wavenumbers g SX_K .. of all three components in
+// is formed once per cell (one reciprocal root for the three components: the 256^3 statistics call takes 589 us,
+// with a root and three divisions 672 us, and E errs by 3.92 and 3.91 x 2^-53 at worst); lane l of every warp
+// then owns row l, and warp g accumulates the SX_K wavenumbers g SX_K .. of all three components in
 // registers, so a staged value feeds 2 SX_K FMAs and the twiddles are warp-uniform (broadcast) reads.
-// Bound by the FP64 pipes: 6 (kmax+1) FMAs and a root per cell.  256^3 FP32, kmax = 8: 3.56 ms for one
-// thread per (component, kx, row), which read uncoalesced and formed every root 3 (kmax+1) times.
+// 6 (kmax+1) FP64 FMAs and a root per cell; 256^3 FP32, kmax = 8: 208 us, waiting for fixed latencies and for the
+// chunk's loads at 10 warps per SM (35.6 KB of shared memory and 64 threads a block).  3.56 ms for one thread per
+// (component, kx, row), which read uncoalesced and formed every root 3 (kmax+1) times.
 constexpr int SX_K = 5, SX_WARPS = 4, SX_PITCH = 33;
 template <class R>
 __global__ void __launch_bounds__(32 * SX_WARPS) spec_x_kernel(const CPlanes<R> u, int nx, size_t rows, int K1,

@@ -294,7 +294,7 @@ class Solver:
 
 
 class Ensemble:
-    """Many periodic GLM boxes of different sizes advanced together, every box on a stream of its own with
+    """Many periodic GLM boxes of different sizes advanced together on the ensemble's own streams, every box with
     its own dt, forcing amplitude and seed (gmt_ensemble_*)."""
 
     def __init__(self, sizes, *, amps=None, seeds=None, dtype="f32", recon="mc", riemann="hlld", gamma=5.0 / 3.0,

@@ -107,6 +107,12 @@ int gmt_destroy(gmt_ctx* ctx);
  * where the FP64 unsplit step runs as passes) */
 int gmt_kernel_info(gmt_ctx* ctx, int32_t* regs, int64_t* smem_bytes, int32_t tile[3]);
 
+/* Overlap.  Steps of one context may run on several streams and be issued by several threads where they share
+ * nothing but the context's tables: unsplit steps and march steps without species, without want_cfl, between
+ * changes of the forcing.  (FP64 unsplit steps take the scratch of their passes in turn, one after another on
+ * the device.)  A context has one pair of CFL words, one loop and forcing record, and one scratch for CT, for
+ * species, for the adjoint and for the statistics: calls that use the same one must be ordered by the caller. */
+
 /* --- GLM step (unsplit: step_plm!/step_tiled!/step_multi!; march1d: march_run_dev) ------- */
 /* uold/unew: base pointers of 9 contiguous planes (plane stride nx*ny*nz), 9 + nsp with species */
 int gmt_step(gmt_ctx* ctx, const void* uold, void* unew, const gmt_step_args* a, void* stream);
@@ -141,10 +147,10 @@ int gmt_run(gmt_ctx* ctx, void* u, void* w, int32_t nsteps, double t0, double t_
 
 /* --- batched ensemble: many periodic boxes of different sizes advanced together
  * (no counterpart in the reference).  Every box: its own n^3 grid (n a multiple of 16), forcing
- * amplitude and seed; the physics of `base`.  Each box advances on a stream of its own, forked from
- * the caller's: a tick, the conditional forcing update and its step kernel per step, ordered only
- * after the box's own previous step, so the boxes fill the chip together.  An FP64 ensemble takes up to
- * 1 GB of scratch for its steps. */
+ * amplitude and seed; the physics of `base`.  The boxes advance on streams forked from the caller's, 64
+ * in FP32 and up to four in FP64, which boxes share in turn where there are more: a tick, the
+ * conditional forcing update and its step kernel per step, ordered only after the stream's earlier work, so
+ * the boxes fill the chip together.  An FP64 ensemble takes up to 1 GB of scratch for its steps. */
 typedef struct gmt_ensemble gmt_ensemble;
 int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, const double* turb_amp,
                         const uint32_t* seeds, gmt_ensemble** out);
