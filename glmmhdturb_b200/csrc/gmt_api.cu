@@ -1203,7 +1203,12 @@ struct gmt_ensemble {
     int nbox = 0;
     int esize = 4;
     std::vector<int> n, ox, lz;      // per box: grid size, tile width, z chunk
-    std::vector<int> order;          // boxes, the longest blocks first: box order[j] runs on lane j % lanes
+    size_t zones = 0;                // of all boxes
+    // boxes, the longest blocks first, and a box's place there: loop, loopc, cfl, modes and bt are in that order
+    std::vector<int> order, place;
+    // what is launched together, boxes order[first] .. order[first + count - 1]: unit j runs on lane j % lanes
+    struct Unit { int first, count; };
+    std::vector<Unit> units;
     std::vector<double> amp;
     std::vector<uint32_t> seed;
     LoopState* loop = nullptr;       // [nbox]
@@ -1273,6 +1278,19 @@ void ens_tiles(gmt_ensemble* E) {
     std::stable_sort(E->order.begin(), E->order.end(), [&](int a, int b) {
         return E->lz[a] != E->lz[b] ? E->lz[a] > E->lz[b] : E->n[a] > E->n[b];
     });
+    E->place.resize(nb);
+    for (int r = 0; r < nb; ++r) E->place[E->order[r]] = r;
+}
+
+// Boxes that are launched each by itself, or, small ones of a size, together (batch_kernel)
+void ens_units(gmt_ensemble* E) {
+    E->units.clear();
+    for (int r = 0, count; r < E->nbox; r += count) {
+        const int n = E->n[E->order[r]];
+        for (count = 1; r + count < E->nbox && E->n[E->order[r + count]] == n; ++count) {}
+        count = std::min(count, ens_batch(E->esize, n, count, E->zones / E->nbox));
+        E->units.push_back({r, count});
+    }
 }
 
 template <class R> void ens_bind(gmt_ensemble* E, void* const* u, void* const* w, int flags) {
@@ -1293,11 +1311,11 @@ template <class R> void ens_bind(gmt_ensemble* E, void* const* u, void* const* w
             a.btab = a.do_turb ? static_cast<const R*>(E->btab[b]) : nullptr;
             a.trigx = static_cast<const R*>(E->trig[3 * b]);
             a.trig8 = static_cast<const R*>(E->trig8[b]);
-            a.cfl_out = E->cfl + 2 * b;
+            a.cfl_out = E->cfl + 2 * E->place[b];
             a.err = E->err;
             a.wait_cycles = GMT_WAIT_CYCLES;
             a.dx = (R)(E->p.boxlen / n);
-            a.dparams = reinterpret_cast<const double*>(E->loop + b);
+            a.dparams = reinterpret_cast<const double*>(E->loop + E->place[b]);
             set_staging(a);
         }
 }
@@ -1308,6 +1326,25 @@ cudaError_t ens_launch(gmt_ensemble* E, const UnsplitArgs<float>& A, int, int, i
 cudaError_t ens_launch(gmt_ensemble* E, const UnsplitArgs<double>& A, int box, int lane, int riem, cudaStream_t s) {
     if (E->pass[lane] && E->pass_S[box] > 0) return launch_passes(A, E->p.recon, riem, E->pass[lane], E->pass_S[box], s);
     return launch_unsplit(A, E->p.recon, riem, s);
+}
+// the boxes of a unit in one launch; A: the boxes' arguments of a parity
+template <class R>
+cudaError_t ens_launch_batch(gmt_ensemble* E, const UnsplitArgs<R>* A, const gmt_ensemble::Unit& U, int riem, cudaStream_t s) {
+    static_assert(sizeof(LoopState) % sizeof(double) == 0, "step values are addressed in doubles");
+    BatchArgs<R> P{};
+    P.A = A[E->order[U.first]];
+    P.chunks = (P.A.nz + P.A.lz - 1) / P.A.lz;
+    P.loop_stride = (int)(sizeof(LoopState) / sizeof(double));
+    P.loop = reinterpret_cast<const double*>(E->loop + U.first);
+    P.cfl = E->cfl + 2 * U.first;
+    for (int i = 0; i < U.count; ++i) {
+        const UnsplitArgs<R>& a = A[E->order[U.first + i]];
+        P.u[i] = a.u.p[0];
+        P.o[i] = a.o.p[0];
+        P.btab[i] = a.btab;
+        P.A.quad = P.A.quad && a.quad;
+    }
+    return launch_batch(P, U.count, E->p.recon, riem, s);
 }
 
 // f() puts the boxes' work on the lanes, which are forked from s and joined to it again
@@ -1324,27 +1361,28 @@ template <class F> cudaError_t ens_fork(gmt_ensemble* E, cudaStream_t s, F f) {
     return e;
 }
 
-// One step of every box, each on its lane and ordered only after that box's own previous step: the boxes
+// One step of every box, each unit on its lane and ordered only after that lane's own earlier work: the boxes
 // are independent, so no box waits for the slowest one and the chip is short of blocks only at the end
 // of a run, not of every step.
 // With `first`, a box's own CFL reduction of its state u[b] goes ahead of its step.
 template <class R> cudaError_t ens_enqueue(gmt_ensemble* E, int par, int flags, bool first) {
     const int riem = E->p.riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : E->p.riemann, L = (int)E->lane.size();
-    const std::vector<UnsplitArgs<R>>& A = ens_args(E, R(0));
+    const UnsplitArgs<R>* A = ens_args(E, R(0)).data() + (size_t)par * E->nbox;
     cudaError_t e = cudaSuccess;
-    for (int j = 0; e == cudaSuccess && j < E->nbox; ++j) {
-        const int b = E->order[j];
-        const cudaStream_t s = E->lane[j % L];
-        if (first) {
-            const UnsplitArgs<R>& a = A[par * E->nbox + b];
-            e = launch_cfl<R>(a.u, (size_t)a.nx * a.ny * a.nz, a.K, E->cfl + 2 * b, s);
-            if (e != cudaSuccess) break;
+    for (size_t j = 0; e == cudaSuccess && j < E->units.size(); ++j) {
+        const gmt_ensemble::Unit U = E->units[j];
+        const int r = U.first, lane = (int)(j % L), n = E->n[E->order[r]];
+        const cudaStream_t s = E->lane[lane];
+        for (int i = r; first && e == cudaSuccess && i < r + U.count; ++i) {
+            const UnsplitArgs<R>& a = A[E->order[i]];
+            e = launch_cfl<R>(a.u, (size_t)n * n * n, a.K, E->cfl + 2 * i, s);
         }
-        tick_kernel<<<1, 64, 0, s>>>(E->loop + b, E->loopc + b, E->cfl + 2 * b, E->modes + (size_t)b * NMODES * 6, E->mode_k_dev);
+        if (e != cudaSuccess) break;
+        tick_kernel<<<U.count, 64, 0, s>>>(E->loop + r, E->loopc + r, E->cfl + 2 * r, E->modes + (size_t)r * NMODES * 6, E->mode_k_dev);
         if (flags & GMT_RUN_FORCING)
-            btab_cond_kernel<R><<<std::min((E->n[b] * E->n[b] + BTAB_ROWS - 1) / BTAB_ROWS, 32), 4 * BTAB_ROWS, 0, s>>>(
-                (const BoxTables<R>*)E->bt + b, E->loop + b, E->mode_k_dev);
-        e = ens_launch(E, A[par * E->nbox + b], b, j % L, riem, s);
+            btab_cond_kernel<R><<<dim3(std::min((n * n + BTAB_ROWS - 1) / BTAB_ROWS, 32), U.count), 4 * BTAB_ROWS, 0, s>>>(
+                (const BoxTables<R>*)E->bt + r, E->loop + r, E->mode_k_dev);
+        e = U.count > 1 ? ens_launch_batch<R>(E, A, U, riem, s) : ens_launch(E, A[E->order[r]], E->order[r], lane, riem, s);
     }
     return e;
 }
@@ -1427,8 +1465,22 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
         if (E->esize == 4) A(&E->trig8[b], (size_t)8 * n[b] * 4);
     }
 
+    for (int b = 0; b < nbox; ++b) E->zones += (size_t)n[b] * n[b] * n[b];
     ens_tiles(E);
-    const int lanes = E->esize == 8 ? pass_lanes(nbox, *std::max_element(n, n + nbox)) : std::min(nbox, ENS_LANES);
+    ens_units(E);
+    const int units = (int)E->units.size();
+    const int lanes = E->esize == 8 ? pass_lanes(units, E->zones / nbox) : std::min(units, ENS_LANES);
+    for (const gmt_ensemble::Unit& U : E->units)
+        if (U.count > 1 && e == cudaSuccess) {
+            if (E->esize == 8) {
+                BatchArgs<double> P{};
+                e = launch_batch(P, 0, base->recon, base->riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : base->riemann, 0);
+            } else {
+                BatchArgs<float> P{};
+                P.A.ox = E->ox[E->order[U.first]];
+                e = launch_batch(P, 0, base->recon, base->riemann == GMT_RIEMANN_LLF ? GMT_RIEMANN_HLLD : base->riemann, 0);
+            }
+        }
     E->lane.assign(lanes, nullptr);
     E->lane_ev.assign(lanes, nullptr);
     for (int i = 0; i < lanes; ++i) {
@@ -1479,15 +1531,16 @@ int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, 
         gmt_params pb = *base;
         pb.nx = pb.ny = pb.nz = n[b];
         pb.turb_seed = E->seed[b];
-        Cs[b] = loop_const_of(pb, alpha, beta, forcing_sigma0(E->amp[b], alpha, beta),
+        const int r = E->place[b];
+        Cs[r] = loop_const_of(pb, alpha, beta, forcing_sigma0(E->amp[b], alpha, beta),
                               GMT_RUN_CH_MAXSIGNAL | GMT_RUN_FORCING);
-        S[b] = LoopState{};
-        S[b].ch = 1.0; S[b].glm_fac = 1.0;
-        S[b].t = 0.0; S[b].t_end = 0.0; S[b].next_time = 0.0; S[b].counter = 0;
-        const double* mb = E->modes + (size_t)b * NMODES * 6;
-        Td[b] = BoxTables<double>{mb, (const double*)E->trig[3 * b + 1], (const double*)E->trig[3 * b + 2],
+        S[r] = LoopState{};
+        S[r].ch = 1.0; S[r].glm_fac = 1.0;
+        S[r].t = 0.0; S[r].t_end = 0.0; S[r].next_time = 0.0; S[r].counter = 0;
+        const double* mb = E->modes + (size_t)r * NMODES * 6;
+        Td[r] = BoxTables<double>{mb, (const double*)E->trig[3 * b + 1], (const double*)E->trig[3 * b + 2],
                                   (double*)E->btab[b], n[b], n[b]};
-        Tf[b] = BoxTables<float>{mb, (const float*)E->trig[3 * b + 1], (const float*)E->trig[3 * b + 2],
+        Tf[r] = BoxTables<float>{mb, (const float*)E->trig[3 * b + 1], (const float*)E->trig[3 * b + 2],
                                  (float*)E->btab[b], n[b], n[b]};
     }
     if (e == cudaSuccess) e = cudaMemcpy(E->loop, S.data(), nbox * sizeof(LoopState), cudaMemcpyHostToDevice);
@@ -1545,9 +1598,7 @@ int gmt_ensemble_run(gmt_ensemble* E, void* const* u, void* const* w, int32_t ns
         return e;
     };
     // A replayed pair of steps pays where launching them one by one takes longer than running them.
-    size_t zones = 0;
-    for (int n : E->n) zones += (size_t)n * n * n;
-    const int pairs = (flags & GMT_RUN_GRAPH) && zones < ENS_GRAPH_ZONES * (size_t)nb ? (nsteps - 1) / 2 : 0;
+    const int pairs = (flags & GMT_RUN_GRAPH) && E->zones < ENS_GRAPH_ZONES * (size_t)nb ? (nsteps - 1) / 2 : 0;
     if (pairs > 0 && !E->exec) {   // from an odd step on: the first one runs by itself, with its CFL
         cudaGraph_t graph;
         GMT_CUDA(cudaStreamBeginCapture(E->cap, cudaStreamCaptureModeRelaxed));
@@ -1573,7 +1624,7 @@ int gmt_ensemble_run(gmt_ensemble* E, void* const* u, void* const* w, int32_t ns
     GMT_CUDA(cudaStreamSynchronize(s));
     int bad = 0;
     for (int b = 0; b < nb; ++b) {
-        if (t_out) t_out[b] = S[b].t;
+        if (t_out) t_out[b] = S[E->place[b]].t;
         bad |= S[b].status;
     }
     if (herr) {

@@ -18,6 +18,11 @@ cudaError_t launch_unsplit(const UnsplitArgs<double>& A, int recon, int riem, cu
 // the FP64 step as three passes over z slabs of S planes with caller-supplied scratch
 cudaError_t launch_passes(const UnsplitArgs<double>& A, int recon, int riem, void* scratch, int S, cudaStream_t s);
 int passes_regs(int recon, int riem);
+// several boxes of one size in one launch (boxes = 0: only sets the kernel's attributes); the schemes of an
+// ensemble, tiles 16x16 and in FP32 32x16 that divide the box
+template <class R> struct BatchArgs;
+cudaError_t launch_batch(const BatchArgs<float>& P, int boxes, int recon, int riem, cudaStream_t s);
+cudaError_t launch_batch(const BatchArgs<double>& P, int boxes, int recon, int riem, cudaStream_t s);
 size_t passes_smem();
 int unsplit_max_threads(int dtype_bytes);
 cudaError_t unsplit_prepare_f32();   // shared-memory attributes of every step kernel

@@ -1,6 +1,7 @@
 // gmt_plan.h -- how a step is cut up for its grid: rules of sizes only, plain C++ without CUDA.
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <cstddef>
 
 namespace gmt {
@@ -33,12 +34,13 @@ inline int pass_slab(int nx, int ny, int nz, size_t budget) {
 }
 
 // Lanes (streams with scratch of their own) of an FP64 ensemble: four, or two where a fourth of the budget
-// would cut the largest box into slabs.  ms a step with 1, 2, 4, 8, 16 lanes: 16 boxes of 32^3 1.59, 0.86,
+// would cut a box of the mean size into slabs.  ms a step with 1, 2, 4, 8, 16 lanes: 16 boxes of 32^3 1.59, 0.86,
 // 0.52, 0.40, 0.39; 8 of 96^3 3.80, 3.49, 3.54, 3.55, 3.56; cut into slabs from four lanes on, 6 of 128^3 6.57,
-// 6.09, 6.32, 6.33, 6.34, and 4 of 192^3 13.96, 13.58, 14.07, 14.08, 14.09 (two slabs with two lanes).
-inline int pass_lanes(int nbox, int largest) {
-    const int lanes = std::min(nbox, 4);
-    return passes_scratch_bytes(largest, largest, largest) <= PASS_SCRATCH_BYTES / lanes ? lanes : std::min(nbox, 2);
+// 6.09, 6.32, 6.33, 6.34, and 4 of 192^3 13.96, 13.58, 14.07, 14.08, 14.09 (two slabs with two lanes).  Small
+// boxes beside large ones need the four: 60 of 32^3 and 4 of 128^3 7.28 with two, 5.98 with four.
+inline int pass_lanes(int units, size_t mean_zones) {
+    const int n = (int)std::cbrt((double)mean_zones), lanes = std::min(units, 4);
+    return passes_scratch_bytes(n, n, n) <= PASS_SCRATCH_BYTES / lanes ? lanes : std::min(units, 2);
 }
 
 // planes per block of the flux pass over a slab of S planes: the extra z face of a chunk costs a third of a
@@ -48,6 +50,21 @@ inline int pass_flux_planes(int nx, int ny, int S) {
     int lz = S;
     while (lz > 4 && bx * by * ((S + lz - 1) / lz) < 148L * PASS_MINB * 3) lz = (lz + 1) / 2;
     return lz;
+}
+
+// --- ensembles -----------------------------------------------------------------------------------
+// How many of `count` boxes of n^3 one launch takes: small boxes by the dozen finish sooner than a launch, a tick
+// and a table for each of them can be started (us a step, own launches -> together, and a persistent kernel
+// over a queue of all boxes' tiles: FP32 512 of 16^3 1297 -> 413, 713; 64 and 256 of 32^3 342 -> 280, 286, and 1231
+// -> 888, 1068; FP64 256 of 16^3 6075 -> 1017, 1439).
+// FP32: 16^3 and 32^3, in ensembles whose mean box is below 40^3.  Among larger boxes the small ones fill gaps
+// better one by one (mean box 79k zones 132 -> 141, 132k 506 -> 550; 73k 441 -> 417; 64 uneven boxes of 642k 15.67 -> 15.99 ms).
+// FP64: 16^3, more of them than lanes (4 of them 99 -> 149, 16 372 -> 152); one by one they run as passes, together
+// as the tile march, whose bits are the same, and 32^3 boxes are faster as passes.
+constexpr int BATCH_BOXES = 64;
+inline int ens_batch(int esize, int n, int count, size_t mean_zones) {
+    const bool small = esize == 8 ? n <= 16 && count > 4 : n <= 32 && mean_zones < (size_t)40 * 40 * 40;
+    return small ? std::min(count, BATCH_BOXES) : 1;
 }
 
 // --- z chunks of the tile marches ----------------------------------------------------------------

@@ -23,6 +23,7 @@
 // forcing kick; the streaming order follows integrator_stream! (:1842-1946).
 #pragma once
 #include "gmt_common.cuh"
+#include "gmt_plan.h"
 
 namespace gmt {
 
@@ -662,6 +663,40 @@ __global__ void __launch_bounds__(MAXT, MINB) unsplit_kernel(const __grid_consta
     extern __shared__ __align__(128) unsigned char smem_raw[];
     scheme_tile<R, UnsplitScheme<R, RECON, RIEM>, TOX, TOY, OVER>(A, step_vals(A), blockIdx.x, blockIdx.y,
                                                                                 blockIdx.z, smem_raw);
+}
+
+// One step of several small boxes of one size (an ensemble's), which the tile divides: blockIdx.z runs over the
+// chunks of all of them.  A box's arrays are kernel parameters at an index that follows from blockIdx, so the
+// tile reads them from constant memory at uniform addresses (128 registers without spills in FP32 MC, as the
+// kernel of one box).  ens_batch says which boxes, with both sides measured.
+template <class R> struct BatchArgs {
+    UnsplitArgs<R> A;       // what the boxes share; u, o, btab, cfl_out and dparams are set per box
+    int chunks;             // z chunks of a box
+    int loop_stride;        // doubles between two boxes' step values
+    const double* loop;     // step values of the first box
+    unsigned long long* cfl;
+    const R* u[BATCH_BOXES];
+    R* o[BATCH_BOXES];
+    const R* btab[BATCH_BOXES];
+};
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX, int TOY>
+__global__ void __launch_bounds__(MAXT, MINB) batch_kernel(const __grid_constant__ BatchArgs<R> P) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int b = blockIdx.z / P.chunks;
+    UnsplitArgs<R> A = P.A;
+    const size_t cells = (size_t)A.nx * A.ny * A.nz;
+#pragma unroll
+    for (int v = 0; v < 9; ++v) {
+        A.u.p[v] = P.u[b] + v * cells;
+        A.o.p[v] = P.o[b] + v * cells;
+    }
+    A.btab = P.btab[b];
+    A.cfl_out = P.cfl + 2 * b;
+    A.dparams = P.loop + (size_t)P.loop_stride * b;
+    A.use_tma = 0;          // boxes this small have no tile clear of their edges
+    A.wait_test = 0;
+    scheme_tile<R, UnsplitScheme<R, RECON, RIEM>, TOX, TOY, false>(A, step_vals(A), blockIdx.x, blockIdx.y,
+                                                                   blockIdx.z - b * P.chunks, smem_raw);
 }
 
 // Tiled march step (the scheme behind march_run_dev); RECON is RECON_MC or RECON_PPM.

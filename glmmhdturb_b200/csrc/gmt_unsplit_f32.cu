@@ -24,6 +24,15 @@ cudaError_t launch_unsplit(const UnsplitArgs<float>& A, int recon, int riem, cud
     if (A.ox * A.oy > 256) return unsplit_dispatch_t<float, 512, 1>(A, recon, riem, s);
     return unsplit_dispatch_t<float, 256, 2>(A, recon, riem, s);
 }
+cudaError_t launch_batch(const BatchArgs<float>& P, int boxes, int recon, int riem, cudaStream_t s) {
+#define GMT_CASE(RC, RM)                                                                           \
+    if (recon == RC && riem == RM)                                                                 \
+        return P.A.ox == 16 ? batch_go<float, RC, RM, 256, 2, 16, 16>(P, boxes, s)                 \
+                            : batch_go<float, RC, RM, 512, 1, 32, 16>(P, boxes, s);
+    GMT_CASE(RECON_MC, RIEM_HLLD) GMT_CASE(RECON_MC, RIEM_HLL) GMT_CASE(RECON_PPM, RIEM_HLL)
+#undef GMT_CASE
+    return cudaErrorNotSupported;
+}
 cudaError_t unsplit_prepare_f32() {
     cudaError_t e = unsplit_configure_all_t<float, 256, 2>();
     if (e == cudaSuccess) e = unsplit_configure_all_t<float, 512, 1>();

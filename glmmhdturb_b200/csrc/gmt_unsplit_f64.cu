@@ -22,6 +22,13 @@ cudaError_t launch_unsplit(const UnsplitArgs<double>& A, int recon, int riem, cu
     if (fixed_tile64<32, 8, false>(A, recon, riem, s, e) || fixed_tile64<16, 16, true>(A, recon, riem, s, e)) return e;
     return unsplit_dispatch_t<double, 256, 1>(A, recon, riem, s);
 }
+cudaError_t launch_batch(const BatchArgs<double>& P, int boxes, int recon, int riem, cudaStream_t s) {
+#define GMT_CASE(RC, RM) \
+    if (recon == RC && riem == RM) return batch_go<double, RC, RM, 256, 1, 16, 16>(P, boxes, s);
+    GMT_CASE(RECON_MC, RIEM_HLLD) GMT_CASE(RECON_MC, RIEM_HLL) GMT_CASE(RECON_PPM, RIEM_HLL)
+#undef GMT_CASE
+    return cudaErrorNotSupported;
+}
 // The step as three passes over z slabs of S planes (gmt_passes.cuh); scratch of passes_scratch_bytes.
 constexpr int PTX = PASS_TX, PTY = PASS_TY, PMINB = PASS_MINB;
 template <int RECON, int RIEM>

@@ -64,6 +64,21 @@ static cudaError_t unsplit_go(const UnsplitArgs<R>& A, cudaStream_t s) {
     return unsplit_run<R, RECON, RIEM, MAXT, MINB, TOX, TOY, TOX == 0>(&A, s, false);
 }
 
+template <class R, int RECON, int RIEM, int MAXT, int MINB, int TOX, int TOY>
+static cudaError_t batch_go(const BatchArgs<R>& P, int boxes, cudaStream_t s) {
+    auto k = batch_kernel<R, RECON, RIEM, MAXT, MINB, TOX, TOY>;
+    static int configured[64] = {0};
+    {
+        cudaError_t e = configure_once(k, configured);
+        if (e != cudaSuccess) return e;
+    }
+    if (boxes <= 0) return cudaSuccess;
+    if (boxes > BATCH_BOXES || P.A.ox != TOX || P.A.oy != TOY || overhangs(P.A)) return cudaErrorInvalidConfiguration;
+    dim3 grid(P.A.nx / TOX, P.A.ny / TOY, P.chunks * boxes);
+    k<<<grid, TOX * TOY, unsplit_smem_bytes<R>(TOX, TOY), s>>>(P);
+    return cudaGetLastError();
+}
+
 template <class R, int MAXT, int MINB>
 static cudaError_t unsplit_dispatch_t(const UnsplitArgs<R>& A, int recon, int riem, cudaStream_t s) {
 #define GMT_CASE(RC, RM) \

@@ -150,7 +150,7 @@ int gmt_run(gmt_ctx* ctx, void* u, void* w, int32_t nsteps, double t0, double t_
  * amplitude and seed; the physics of `base`.  The boxes advance on streams forked from the caller's, 64
  * in FP32 and up to four in FP64, which boxes share in turn where there are more: a tick, the
  * conditional forcing update and its step kernel per step, ordered only after the stream's earlier work, so
- * the boxes fill the chip together.  An FP64 ensemble takes up to 1 GB of scratch for its steps. */
+ * the boxes fill the chip together; many small boxes of one size share these launches.  An FP64 ensemble takes up to 1 GB of scratch for its steps. */
 typedef struct gmt_ensemble gmt_ensemble;
 int gmt_ensemble_create(const gmt_params* base, int32_t nbox, const int32_t* n, const double* turb_amp,
                         const uint32_t* seeds, gmt_ensemble** out);

@@ -1,6 +1,6 @@
 """Ensembles whose boxes share a stream (more boxes than lanes: 64 in FP32, 4 or 2 in FP64, where a lane's boxes also
-take its scratch in turn), runs without and with the replayed pair of steps, odd and even numbers of
-steps, and a box of several slabs.  Every box must equal its own single-box run."""
+take its scratch in turn) or a launch (small boxes of one size), runs without and with the replayed pair of
+steps, odd and even numbers of steps, and a box of several slabs.  Every box must equal its own single-box run."""
 import pytest
 import torch
 
@@ -11,16 +11,16 @@ pytestmark = pytest.mark.gpu
 COURANT, CP, T = 0.3, 0.18, 0.5
 
 
-def _runs(sizes, dtype, steps, graph=True):
+def _runs(sizes, dtype, steps, graph=True, **scheme):
     """The ensemble's states and times after `steps` steps, and each box's from a single-box run."""
     from glmmhdturb_b200 import Ensemble, Solver
     amps, seeds = [1.0 + 0.25 * (b % 7) for b in range(len(sizes))], [11 + b for b in range(len(sizes))]
-    ens = Ensemble(sizes, amps=amps, seeds=seeds, dtype=dtype, courant=COURANT, turb_T=T, glm_cp_coef=CP)
+    ens = Ensemble(sizes, amps=amps, seeds=seeds, dtype=dtype, courant=COURANT, turb_T=T, glm_cp_coef=CP, **scheme)
     u, w = ens.alloc(), ens.alloc()
     singles = []
     for b, n in enumerate(sizes):
         s = Solver(n, dtype=dtype, gamma=5 / 3, courant=COURANT, turb_amp=amps[b], turb_T=T, turb_ndt=100, turb_seed=seeds[b],
-                   glm_cp_coef=CP)
+                   glm_cp_coef=CP, **scheme)
         s.ic_turbulent(u[b], mach=0.5 + 0.1 * (b % 6), seed=seeds[b])
         x, y = u[b].clone(), torch.empty_like(u[b])
         s.forcing_reset()
@@ -39,7 +39,7 @@ def test_fp64_boxes_share_lanes_and_their_scratch(steps):
 
 
 def test_fp64_box_of_several_slabs_beside_others():
-    """On two lanes a 160^3 box has two slabs; the mean box is above 48^3, so no steps are replayed."""
+    """With four lanes a 160^3 box has three slabs; the mean box is above 48^3, so no steps are replayed."""
     t, got, singles = _runs([160, 64, 80, 96, 32], "f64", 3)
     for b, (ts, ref) in enumerate(singles):
         assert t[b] == ts and torch.equal(got[b], ref), b
@@ -62,3 +62,45 @@ def test_fp32_steps_that_are_not_replayed(steps):
 @pytest.mark.parametrize("steps,graph", [(4, True), (5, True), (5, False)])
 def test_fp32_more_boxes_than_lanes(steps, graph):
     _check_f32(*_runs([16, 32, 16, 48, 16] * 14, "f32", steps, graph))
+
+
+# small boxes of one size in one launch: fewer and more than a launch takes (64), beside others; each scheme
+@pytest.mark.parametrize("sizes,steps", [([16] * 5, 3), ([16] * 70 + [32], 4), ([32, 16] * 6, 5)])
+def test_fp64_small_boxes_share_launches(sizes, steps):
+    t, got, singles = _runs(sizes, "f64", steps)
+    for b, (ts, ref) in enumerate(singles):
+        assert t[b] == ts and torch.equal(got[b], ref), b
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("recon,riemann", [("mc", "hll"), ("mc", "llf"), ("ppm", "hll")])
+def test_schemes_of_boxes_that_share_launches(dtype, recon, riemann):
+    t, got, singles = _runs([16] * 6 + [32] * 2, dtype, 3, recon=recon, riemann=riemann)
+    if dtype == "f32":
+        _check_f32(t, got, singles)
+    else:
+        for b, (ts, ref) in enumerate(singles):
+            assert t[b] == ts and torch.equal(got[b], ref), b
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_states_off_a_16_byte_boundary(dtype):
+    """One box of a shared launch whose planes allow no 16-byte copies: the same values as with aligned ones."""
+    from glmmhdturb_b200 import Ensemble, Solver
+    sizes = [16] * 6 + [32] * 3
+    out = []
+    for shift in (0, 1):
+        ens = Ensemble(sizes, amps=[2.0] * len(sizes), dtype=dtype, courant=COURANT, turb_T=T, glm_cp_coef=CP)
+        u, w = ens.alloc(), ens.alloc()
+        for b, n in enumerate(sizes):
+            s = Solver(n, dtype=dtype, gamma=5 / 3)
+            s.ic_turbulent(u[b], mach=0.8, seed=b)
+            s.close()
+        if shift:
+            for b in (2, 7):
+                flat = torch.empty(u[b].numel() + shift, dtype=u[b].dtype, device="cuda")[shift:].view(u[b].shape)
+                u[b] = flat.copy_(u[b])
+        t = ens.run(u, w, 3)
+        out.append((t, w))
+    assert out[0][0] == out[1][0]
+    assert all(torch.equal(a, b) for a, b in zip(out[0][1], out[1][1]))

@@ -58,11 +58,38 @@ def test_fp64_scratch_stays_within_its_budget(plan, n, lanes):
         assert S >= min(3, n[2]) and size <= budget
 
 
-@pytest.mark.parametrize("nbox,largest,lanes", [(1, 192, 1), (2, 256, 2), (3, 128, 3), (4, 112, 4), (64, 32, 4), (4, 128, 2),
-                                                (64, 192, 2), (5, 512, 2)])
-def test_fp64_lanes_keep_boxes_whole_where_two_of_them_can(plan, nbox, largest, lanes):
-    (got,), = plan(("lanes", nbox, largest))
+@pytest.mark.parametrize("units,mean,lanes", [(1, 192 ** 3, 1), (2, 256 ** 3, 2), (3, 128 ** 3, 3), (4, 112 ** 3, 4), (64, 32 ** 3, 4),
+                                              (4, 128 ** 3, 2), (64, 192 ** 3, 2), (64, (60 * 32 ** 3 + 4 * 128 ** 3) // 64, 4)])
+def test_fp64_lanes_keep_a_mean_box_whole_where_two_of_them_can(plan, units, mean, lanes):
+    (got,), = plan(("lanes", units, mean))
     assert got == lanes
+
+
+# dtype, boxes by size, us a step of the ensemble with a launch for each box and with those of a size together
+BATCHES = [
+    ("f32", {16: 64}, 213, 79), ("f32", {16: 512}, 1297, 413), ("f32", {32: 64}, 342, 280), ("f32", {32: 256}, 1231, 888),
+    ("f32", {16: 100, 128: 1}, 514, 328), ("f32", {32: 32, 48: 4}, 256, 231), ("f32", {32: 5, 48: 1}, 79, 72),
+    ("f32", {32: 6, 48: 3, 64: 1}, 132, 141), ("f32", {32: 14, 48: 8, 64: 12}, 506, 550), ("f32", {32: 8, 64: 8}, 254, 279),
+    ("f32", {32: 13, 48: 13, 64: 12, 96: 13, 128: 13}, 4025, 4093), ("f32", {48: 64}, 798, 794),
+    ("f64", {16: 4}, 99, 149), ("f64", {16: 16}, 372, 152), ("f64", {16: 256}, 6075, 1017), ("f64", {16: 100, 128: 1}, 5731, 2191),
+    ("f64", {16: 3, 256: 1}, 8740, 9217),
+]
+
+
+@pytest.mark.parametrize("dtype,boxes,alone,together", BATCHES)
+def test_small_boxes_share_launches_where_that_is_faster(plan, dtype, boxes, alone, together):
+    """Boxes of 16^3 (and in FP32 of 32^3) share launches where the ensemble was measured faster by more than 3 % for
+    it, and do not where it was slower by as much as 1 %."""
+    mean = sum(c * n ** 3 for n, c in boxes.items()) // sum(boxes.values())
+    esize = 8 if dtype == "f64" else 4
+    got = {n: c for n, (c,) in zip(boxes, plan(*[("batch", esize, n, c, mean) for n, c in boxes.items()]))}
+    assert all(1 <= got[n] <= min(c, 64) for n, c in boxes.items())
+    assert all(c == 1 for n, c in got.items() if n > (16 if dtype == "f64" else 32))
+    shares = max(got.values()) > 1
+    if together < 0.97 * alone:
+        assert shares
+    if together > 1.01 * alone:
+        assert not shares
 
 
 # us a step of a tile march: with the rule that asked for eight rounds of blocks and no more (the kernels of
