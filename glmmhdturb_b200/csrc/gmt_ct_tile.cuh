@@ -73,24 +73,29 @@ __device__ __forceinline__ void ct_stage_plane(R* __restrict__ SG, const CPlanes
                                                int nt) {
     constexpr int Q = 16 / (int)sizeof(R);
     const size_t nxy = (size_t)nx * ny, plane = nxy * wrapi(kp, nz), plane1 = nxy * wrapi(kp + 1, nz);
-    if (ROWS || al16) {
-        const int qw = SW / Q, jobs = qw * (SN5 / SW);
-        for (int j = tid; j < jobs; j += nt) {
-            const int row = j / qw, col = (j % qw) * Q;
+    if (ROWS) {
+        const int step = al16 ? Q : 1;
+        for (int c = tid * step; c < SN5; c += nt * step) {
+            const int row = c / SW, col = c % SW;
             const size_t gxy = (size_t)wrapi(x0 - 4 + col, nx) + (size_t)nx * wrapi(y0 - 2 + row, ny);
-            const int cs = row * SW + col;
             if (al16) {
 #pragma unroll
-                for (int v = 0; v < 8; ++v) cp_async16(SG + v * SN5 + cs, q.p[v] + plane + gxy);
-                cp_async16(SG + 8 * SN5 + cs, q.p[7] + plane1 + gxy);
-            } else {
-#pragma unroll 1
-                for (int i = 0; i < Q; ++i) {
+                for (int v = 0; v < 8; ++v) cp_async16(SG + v * SN5 + c, q.p[v] + plane + gxy);
+                cp_async16(SG + 8 * SN5 + c, q.p[7] + plane1 + gxy);
+            } else if (col >= 2 && col < SW - 1) {
 #pragma unroll
-                    for (int v = 0; v < 8; ++v) cp_async_r(SG + v * SN5 + cs + i, q.p[v] + plane + gxy + i);
-                    cp_async_r(SG + 8 * SN5 + cs + i, q.p[7] + plane1 + gxy + i);
-                }
+                for (int v = 0; v < 8; ++v) cp_async_r(SG + v * SN5 + c, q.p[v] + plane + gxy);
+                cp_async_r(SG + 8 * SN5 + c, q.p[7] + plane1 + gxy);
             }
+        }
+    } else if (al16) {
+        const int qw = SW / Q, jobs = qw * (SN5 / SW);
+        for (int j = tid; j < jobs; j += nt) {
+            const int row = j / qw, col = (j % qw) * Q, cs = row * SW + col;
+            const size_t gxy = (size_t)wrapi(x0 - 4 + col, nx) + (size_t)nx * wrapi(y0 - 2 + row, ny);
+#pragma unroll
+            for (int v = 0; v < 8; ++v) cp_async16(SG + v * SN5 + cs, q.p[v] + plane + gxy);
+            cp_async16(SG + 8 * SN5 + cs, q.p[7] + plane1 + gxy);
         }
     } else {
         for (int c = tid; c < PN5; c += nt) {
@@ -295,7 +300,7 @@ __device__ __forceinline__ void ct_tile(const CTArgs<R>& A, int bx, int by, int 
             }
             if (!tma && !A.wait_test) {
                 ct_stage_plane<!OVER>(SG, A.q, quad, PN5, PW5, SW, SN5, x0, y0, kr + 2, nx, ny, nz,
-                               tid >= stg0 ? tid - stg0 : INT_MAX, NT - stg0);
+                               tid >= stg0 ? tid - stg0 : (OVER ? INT_MAX : SN5), NT - stg0);
                 mbar_arrive_cp_async(mbar);
             }
         }

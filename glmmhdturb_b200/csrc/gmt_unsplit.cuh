@@ -157,8 +157,9 @@ __device__ __forceinline__ int mod3(int k) {
 // row pitch SW = OX + 8 and the region starting at column 2: exactly the box (x0-4, y0-2) of
 // (OX+8) x (OY+4) cells that one TMA copy delivers (its first column 16-byte aligned).
 // Rows of whole quads (nx and the tile width multiples of 4, in FP64 of 2): a quad of 16 bytes never
-// straddles the periodic boundary, so the staged rows are copied quad by quad -- one 16-byte copy each,
-// or, where a plane is not 16-byte aligned (al16 false), one copy per cell.  A 4-byte copy per cell costs
+// straddles the periodic boundary, so the staged rows are copied by 16 bytes each, or, where a plane is not
+// 16-byte aligned (al16 false), cell by cell, a warp's lanes on consecutive cells (four of a quad in one lane
+// instead: misaligned 256^3 step 1554 us against 1391).  A 4-byte copy per cell costs
 // every thread of a 32x16 tile 15 copies and their address arithmetic per plane, 4 % of the step's
 // instructions.  ROWS: the tile divides the box, so its rows are known to be whole quads and the
 // cell-by-cell loop for other rows is not compiled in (it took registers from the 128-register tiles
@@ -168,21 +169,26 @@ __device__ __forceinline__ void stage_plane(R* __restrict__ SG, const CPlanes<R>
                                             int SN, int x0, int y0, int kp, int nx, int ny, int nz, int tid, int nt) {
     constexpr int Q = 16 / (int)sizeof(R);
     const size_t plane = (size_t)nx * ny * wrapi(kp, nz);
-    if (ROWS || al16) {
+    if (ROWS) {
+        const int step = al16 ? Q : 1;
+        for (int c = tid * step; c < SN; c += nt * step) {
+            const int row = c / SW, col = c % SW;
+            const size_t g = plane + (size_t)wrapi(x0 - 4 + col, nx) + (size_t)nx * wrapi(y0 - 2 + row, ny);
+            if (al16) {
+#pragma unroll
+                for (int v = 0; v < 9; ++v) cp_async16(SG + v * SN + c, u.p[v] + g);
+            } else if (col >= 2 && col < SW - 2) {
+#pragma unroll
+                for (int v = 0; v < 9; ++v) cp_async_r(SG + v * SN + c, u.p[v] + g);
+            }
+        }
+    } else if (al16) {
         const int qw = SW / Q, jobs = qw * (SN / SW);
         for (int j = tid; j < jobs; j += nt) {
             const int row = j / qw, col = (j % qw) * Q;
             const size_t g = plane + (size_t)wrapi(x0 - 4 + col, nx) + (size_t)nx * wrapi(y0 - 2 + row, ny);
-            const int cs = row * SW + col;
-            if (al16) {
 #pragma unroll
-                for (int v = 0; v < 9; ++v) cp_async16(SG + v * SN + cs, u.p[v] + g);
-            } else {
-#pragma unroll 1
-                for (int i = 0; i < Q; ++i)
-#pragma unroll
-                    for (int v = 0; v < 9; ++v) cp_async_r(SG + v * SN + cs + i, u.p[v] + g + i);
-            }
+            for (int v = 0; v < 9; ++v) cp_async16(SG + v * SN + row * SW + col, u.p[v] + g);
         }
     } else {
         for (int c = tid; c < PN; c += nt) {
@@ -450,7 +456,7 @@ __device__ __forceinline__ void scheme_tile(const UnsplitArgs<R>& A, const StepV
             }
             if (!tma && !A.wait_test) {
                 stage_plane<!OVER>(SG, A.u, quad, PNc, PW, SW, SN, x0, y0, kr + 2, nx, ny, nz,
-                                   tid >= stg0 ? tid - stg0 : INT_MAX, NT - stg0);
+                                   tid >= stg0 ? tid - stg0 : (OVER ? INT_MAX : SN), NT - stg0);
                 mbar_arrive_cp_async(mbar);
             }
         }
