@@ -10,6 +10,7 @@ namespace gmt {
 constexpr int PASS_TX = 16, PASS_TY = 8;   // columns per block of the flux pass
 constexpr int PASS_MINB = 4;               // its blocks on an SM
 constexpr size_t PASS_SCRATCH_BYTES = (size_t)1 << 30;   // of a context, or of all lanes of an ensemble
+constexpr size_t PASS_OVERLAP_ZONES = (size_t)40 * 40 * 40;   // boxes below: steps on several streams overlap
 constexpr int GRID_YZ = 65535;             // largest gridDim.y and gridDim.z
 
 // scratch of a slab of S planes: primitives of S + 4 planes, predictors of S + 2, PPM's flags

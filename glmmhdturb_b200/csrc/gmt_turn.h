@@ -18,12 +18,13 @@ public:
     ScratchTurn(const ScratchTurn&) = delete;
     ScratchTurn& operator=(const ScratchTurn&) = delete;
     cudaError_t status() const { return status_; }
-    // all of the holder's work is on the stream
+    // all of the holder's work is on the stream: the next holder may come
     cudaError_t mark() {
         if (!open_) return cudaSuccess;
         open_ = false;
         const cudaError_t e = cudaEventRecord(ev_, s_);
         if (e != cudaSuccess) cudaStreamSynchronize(s_);
+        lock_.unlock();
         return e;
     }
 

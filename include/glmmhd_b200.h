@@ -110,7 +110,7 @@ int gmt_kernel_info(gmt_ctx* ctx, int32_t* regs, int64_t* smem_bytes, int32_t ti
 /* Overlap.  Steps of one context may run on several streams and be issued by several threads where they share
  * nothing but the context's tables: unsplit steps and march steps without species, without want_cfl, between
  * changes of the forcing.  (FP64 unsplit steps take the scratch of their passes in turn, one after another on
- * the device.)  A context has one pair of CFL words, one loop and forcing record, and one scratch for CT, for
+ * the device; those of boxes below 40^3 run as the tile march instead where the stream changes.)  A context has one pair of CFL words, one loop and forcing record, and one scratch for CT, for
  * species, for the adjoint and for the statistics: calls that use the same one must be ordered by the caller. */
 
 /* --- GLM step (unsplit: step_plm!/step_tiled!/step_multi!; march1d: march_run_dev) ------- */

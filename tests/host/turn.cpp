@@ -47,7 +47,7 @@ int main() {
         mu.unlock();
         std::printf("end\n");
     }
-    // another thread gets its turn only when the first has left
+    // another thread gets its turn only when the first has left, or marked the end of its work
     std::thread t;
     {
         gmt::ScratchTurn turn(mu, nullptr, (cudaStream_t)(intptr_t)1);
@@ -56,6 +56,12 @@ int main() {
         std::printf("launch 1\n");
     }
     t.join();
+    std::printf("end\n");
+    {
+        gmt::ScratchTurn turn(mu, nullptr, (cudaStream_t)(intptr_t)1);
+        turn.mark();
+        std::thread([] { hold(2, false); }).join();
+    }
     std::printf("end\n");
     return 0;
 }

@@ -85,6 +85,31 @@ def test_under_capture_and_after():
     assert torch.equal(x, y)
 
 
+@pytest.mark.parametrize("n", [(24, 24, 24), (33, 20, 9)])
+def test_small_boxes_on_several_streams(n):
+    """Steps of small boxes that change the stream take the march, which overlaps, instead of turns at the
+    scratch; the values are the same in any order of streams, and a stream that stays takes the passes again."""
+    from glmmhdturb_b200 import Solver
+    s = Solver(n, dtype="f64", gamma=5 / 3)
+    us, ref = [], []
+    for seed in range(4):
+        u = s.alloc()
+        s.ic_turbulent(u, mach=1.0, seed=seed + 1)
+        o = torch.empty_like(u)
+        s.step(u, o, 0.02 * s.dx, ch=3.0, glm_fac=0.99)
+        us.append(u)
+        ref.append(o)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in us]
+    outs = [torch.full_like(u, float("nan")) for u in us]
+    torch.cuda.synchronize()
+    for i in (0, 1, 2, 3, 3, 3, 0, 2, 1, 1, 0):
+        s.step(us[i], outs[i], 0.02 * s.dx, ch=3.0, glm_fac=0.99, stream=streams[i])
+    torch.cuda.synchronize()
+    for o, r in zip(outs, ref):
+        assert torch.equal(o, r)
+
+
 def test_two_streams_share_a_context():
     """Steps of one context on two streams take its scratch in turn."""
     from glmmhdturb_b200 import Solver

@@ -154,6 +154,7 @@ def test_scratch_is_handed_on_however_a_holder_leaves(tmp_path):
     assert got[2] == ["wait 1", "status 1", "free 1"]
     assert got[3] == ["wait 1", "launch 1", "record 1", "synchronise 1", "status 1", "free 1"]
     assert got[4] == ["wait 1", "launch 1", "record 1", "wait 2", "launch 2", "record 2"]
+    assert got[5] == ["wait 1", "record 1", "wait 2", "launch 2", "record 2"]
 
 
 def test_tensor_maps_kept_for_later_steps_are_whole(tmp_path):
