@@ -1242,6 +1242,7 @@ struct gmt_ensemble {
     std::vector<const void*> bound_u, bound_w;
     cudaGraphExec_t exec = nullptr;
     int exec_flags = -1;
+    bool ran = false;                // a run on the bound states has been launched
     std::vector<double> alpha, beta, sigma0;
 };
 
@@ -1585,6 +1586,7 @@ int gmt_ensemble_run(gmt_ensemble* E, void* const* u, void* const* w, int32_t ns
         E->bound_w.assign(w, w + nb);
         if (E->exec) { cudaGraphExecDestroy(E->exec); E->exec = nullptr; }
         E->exec_flags = flags;
+        E->ran = false;
         // per-run flags live in the loop constants
         std::vector<LoopConst> Cs(nb);
         GMT_CUDA(cudaMemcpy(Cs.data(), E->loopc, nb * sizeof(LoopConst), cudaMemcpyDeviceToHost));
@@ -1607,8 +1609,12 @@ int gmt_ensemble_run(gmt_ensemble* E, void* const* u, void* const* w, int32_t ns
         for (int i = 0; e == cudaSuccess && i < n; ++i) e = ens_enqueue_any(E, i & 1, flags, start && i == 0);
         return e;
     };
-    // A replayed pair of steps pays where launching them one by one takes longer than running them.
-    const int pairs = (flags & GMT_RUN_GRAPH) && E->zones < ENS_GRAPH_ZONES * (size_t)nb ? (nsteps - 1) / 2 : 0;
+    // A replayed pair of steps pays where launching them one by one takes longer than running them, and from
+    // the second run on the same states on: making the graph takes as long as dozens of steps (21 boxes of 32^3 and 23 of
+    // 48^3: 5 ms, a step 0.45 ms), which a caller who exchanges u and w after an odd run would pay each time.
+    const bool replay = (flags & GMT_RUN_GRAPH) && E->ran && E->zones < ENS_GRAPH_ZONES * (size_t)nb;
+    const int pairs = replay ? (nsteps - 1) / 2 : 0;
+    E->ran = E->ran || nsteps > 0;
     if (pairs > 0 && !E->exec) {   // from an odd step on: the first one runs by itself, with its CFL
         cudaGraph_t graph;
         GMT_CUDA(cudaStreamBeginCapture(E->cap, cudaStreamCaptureModeRelaxed));
